@@ -55,7 +55,6 @@ constexpr int EMAX = 16;
 constexpr size_t ALIGN = 256;
 constexpr int HIST_CAP = 65536;
 constexpr int ELEM_MAX_CTAS = 1184;      // 8 x 148 SMs
-constexpr size_t COL_SMEM_BUDGET = 96 * 1024;
 constexpr int MAX_FFT = 16384;           // longest register FFT (1024 threads x 16)
 // longest transform of the shared-memory FFT (1024 threads x up to 32 elements,
 // one 8-byte slot per element within the 227 KB of shared memory a CTA can have)
@@ -144,14 +143,14 @@ HostPlan make_plan(int N) {
 
 // ------------------------------------------------------------ layout
 struct GridLayout {
-    size_t st, counter, part, tw_r, dw_r, ch_r, hs_r, cos_r, tw_c, dw_c, ch_c, hs_c, cos_c;
+    size_t st, counter, part, tw_r, dw_r, ch_r, hs_r, cos_r, cos_c, tri;
     size_t arr[20];          // gx gy wx wy | wIx wIy b r z p0 p1 Ap T | U0 U1 Ub | L0 L1 Lb D
     size_t valid, hist, tilecnt;
     size_t tc;               // split DCT matrices of the tensor-core column pass (H0 <= UNW_TC_MAX_H), else 0
     size_t post_parent, post_lab, post_csum, post_ccount, post_remap, post_adj;
     size_t end;
     long long P0, max_ctas, lab_cap, ntiles_max;
-    int fr_cap, fc_cap;      // capacities of the FFT tables (row / column)
+    int fr_cap;              // capacity of the FFT tables
 };
 
 struct BatchLayout {
@@ -177,7 +176,6 @@ GridLayout grid_layout(long long H0, long long W0) {
         return std::max<long long>(c, std::min<long long>(MAX_FFT, std::max<long long>(256, next_pow2(2 * N0 - 1))));
     };
     L.fr_cap = (int)cap(W0);
-    L.fc_cap = (int)cap(H0);
     L.st = take(sizeof(InstState));
     L.counter = take(sizeof(unsigned) * 4);
     L.part = take((size_t)L.max_ctas * UNW_NPART * sizeof(double));
@@ -186,11 +184,8 @@ GridLayout grid_layout(long long H0, long long W0) {
     L.dw_r = take(sizeof(float2) * W0);
     L.ch_r = take(sizeof(float2) * W0);
     L.cos_r = take(sizeof(float) * W0);
-    L.tw_c = take(sizeof(float2) * L.fc_cap);
-    L.hs_c = take(sizeof(float2) * L.fc_cap);
-    L.dw_c = take(sizeof(float2) * H0);
-    L.ch_c = take(sizeof(float2) * H0);
     L.cos_c = take(sizeof(float) * H0);
+    L.tri = take(unw_tri_table_bytes(W0));
     for (int a = 0; a < 20; a++) L.arr[a] = take(A);
     L.valid = take((size_t)H0 * L.P0);
     L.tc = H0 <= UNW_TC_MAX_H ? take(unw_tc_table_bytes((int)H0)) : 0;
@@ -236,13 +231,14 @@ BatchLayout batch_layout(int n, const long long* H, const long long* W) {
 
 // ------------------------------------------------------------ launch shapes
 struct Shape {
-    int row_T = 0, col_T = 0;
-    int row_emax = 16, col_emax = 16;   // elements per thread of the shared-memory FFT
-    size_t row_smem = 0, col_smem = 0;
-    int row_p2 = 0, col_p2 = 0;   // power-of-two register-FFT paths (length), 0 = generic
-    int row_bl = 0, col_bl = 0;   // Bluestein register-FFT paths (FFT length M), 0 = not used
+    int row_T = 0;
+    int row_emax = 16;            // elements per thread of the shared-memory FFT
+    size_t row_smem = 0;
+    int row_p2 = 0;               // power-of-two register-FFT path (length), 0 = generic
+    int row_bl = 0;               // Bluestein register-FFT path (FFT length M), 0 = not used
+    int tri_L = 0;                // column pass: rows per segment
+    int tri_tma = 0;              // ... with its tiles moved by TMA
     int col_tc = 0;               // tensor-core column pass (mixed precision), chosen by the autotuner
-    int col_p2_tma = 0;           // power-of-two column pass with the slab moved by TMA (H 2048 / 4096)
     int mv_tma = 0;               // matvec on TMA-staged halo tiles
 };
 
@@ -328,7 +324,7 @@ int kind_ctas(const GridDev& G, int kind) {
     switch (kind) {
         // persistent kinds: at most a few CTAs per SM, each loops over its units
         case KS_ROWPAIR: return std::min((G.H + 1) / 2, CTAS_ROW);
-        case KS_COL: return std::min((G.W + 2 * G.col_nseq - 1) / (2 * G.col_nseq), G.col_ctas);
+        case KS_COL: return G.col_ctas;
         case KS_STEN: return std::min(G.sten_tiles_x * ((G.H + 8 * G.sten_rows - 1) / (8 * G.sten_rows)), CTAS_HEAD);
         case KS_MATVEC: return std::min(G.sten_tiles_x * ((G.H + 15) / 16), CTAS_MATVEC);
         case KS_ELEM: return elem_ctas(npx);
@@ -354,12 +350,8 @@ cudaError_t L_rowi(Solver& S, int mode) {
 }
 cudaError_t L_col(Solver& S, int mode) {
     if (S.sh.col_tc) return unw_launch_col_tc(mode, S.total[KS_TC], S.s, S.dg, S.ds(KS_TC), S.n, &S.maps, S.bmaps);
-    if (S.sh.col_p2_tma)
-        return unw_launch_col_p2_tma(S.sh.col_p2, mode, S.total[KS_COL], S.s, S.dg, S.ds(KS_COL), S.n, S.bmaps);
-    if (S.sh.col_p2) return unw_launch_col_p2(S.sh.col_p2, mode, S.total[KS_COL], S.s, S.dg, S.ds(KS_COL), S.n);
-    if (S.sh.col_bl) return unw_launch_col_bl(S.sh.col_bl, mode, S.total[KS_COL], S.s, S.dg, S.ds(KS_COL), S.n);
-    return unw_launch_col(mode, S.sh.col_T, S.sh.col_emax, S.total[KS_COL], S.sh.col_smem, S.s, S.dg, S.ds(KS_COL),
-                          S.n);
+    return unw_launch_col_tri(S.sh.tri_L, S.sh.tri_tma != 0, mode, S.total[KS_COL], S.s, S.dg, S.ds(KS_COL), S.n,
+                              S.bmaps);
 }
 
 // ------------------------------------------------------------ IRLS enqueue
@@ -488,72 +480,22 @@ int validate_params(const unw_params* p) {
     return UNW_OK;
 }
 
-// column pairs per generic column CTA under the shared-memory budget
-int col_nseq_generic(int nfft, int W) {
-    int nseq = (int)std::max<size_t>(1, std::min<size_t>(8, COL_SMEM_BUDGET / ((size_t)nfft * sizeof(float2))));
-    return std::min(nseq, (W + 1) / 2);
-}
-
 // Launch-group key of a cropped H x W grid: grids with equal keys share every
-// kernel configuration (power-of-two length, or generic thread count) per axis.
-std::array<int, 4> group_key(int H, int W) {
+// kernel configuration: power-of-two length, Bluestein length or generic thread count of the
+// rows, rows per segment of the column pass.
+std::array<int, 4> group_key(int H, int W, int flags) {
     if (H <= 0 || W <= 0) return {-1, 0, -1, 0};
     auto p2 = [](int n) { return n >= 256 && n <= MAX_FFT && (n & (n - 1)) == 0; };
     std::array<int, 4> k{};
     if (p2(W)) { k[0] = 1; k[1] = W; }
     else if (bl_len(W)) { k[0] = 2; k[1] = bl_len(W); }
     else { const HostPlan hp = make_plan(W); k[0] = 0; k[1] = pick_threads(hp.n, hp.cap) * 64 + hp.emax; }
-    if (p2(H)) { k[2] = 1; k[3] = H; }
-    else if (bl_len(H)) { k[2] = 2; k[3] = bl_len(H); }
-    else {
-        const HostPlan hp = make_plan(H);
-        int nseq = col_nseq_generic(hp.n, W), cT = 0;
-        while (nseq >= 1 && !(cT = pick_threads((long long)nseq * hp.n, hp.cap))) nseq--;
-        k[2] = 0; k[3] = cT * 64 + hp.emax;
-    }
+    k[2] = unw_tri_rows(H, W);
+    if (flags & UNW_F_MIXED) k[3] = H;  // the tensor-core column pass needs one H per launch
     return k;
 }
 
-// Autotuner of the power-of-two column pass at H = 2048 / 4096: times the pass with the
-// slab moved by TMA against the plain-load pass on the group's own buffers (DCT
-// initial-solve mode; two warm-up and three timed launches of each on the solve stream)
-// and returns 1 when TMA is faster.  Both give the same bits, so the choice changes only
-// the time.  Cached per device, H and the group's total width for the life of the
-// process; it runs before any graph capture.
-int autotune_tma(Solver& S, int H, int Wsum) {
-    static std::mutex mu;
-    static std::map<std::array<int, 3>, int> cache;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const std::array<int, 3> key{dev, H, Wsum};
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = cache.find(key);
-        if (it != cache.end()) return it->second;
-    }
-    cudaEvent_t e[4];
-    for (auto& x : e) cudaEventCreate(&x);
-    bool ok = true;
-    for (int tma = 0; tma < 2; tma++) {
-        S.sh.col_p2_tma = tma;
-        for (int r = 0; r < 2; r++) ok &= L_col(S, 0) == cudaSuccess;
-        cudaEventRecord(e[2 * tma], S.s);
-        for (int r = 0; r < 3; r++) ok &= L_col(S, 0) == cudaSuccess;
-        cudaEventRecord(e[2 * tma + 1], S.s);
-    }
-    float t_plain = 0.f, t_tma = 0.f;
-    int res = 1;
-    if (ok && cudaEventSynchronize(e[3]) == cudaSuccess && cudaEventElapsedTime(&t_plain, e[0], e[1]) == cudaSuccess &&
-        cudaEventElapsedTime(&t_tma, e[2], e[3]) == cudaSuccess)
-        res = t_tma < t_plain ? 1 : 0;
-    cudaGetLastError();
-    for (auto& x : e) cudaEventDestroy(x);
-    std::lock_guard<std::mutex> lk(mu);
-    cache[key] = res;
-    return res;
-}
-
-// Autotuner of the mixed-precision form: times the FFT column pass against the
+// Autotuner of the mixed-precision form: times the default column pass against the
 // tensor-core one on the group's own buffers (DCT initial-solve mode, which has no
 // PCG gate; two warm-up and three timed launches of each on the solve stream) and
 // returns 1 when the tensor cores are faster.  The choice is cached per device and
@@ -611,7 +553,7 @@ int prepare(Solver& S, const std::vector<int>& idx, const unw_grid* grids, const
     S.sc.cg_tol = fixed ? 0.f : prm->cg_tol;  // ||r|| < 0 never holds
     S.sc.eps2 = (float)((double)prm->epsilon * (double)prm->epsilon);
     S.sc.conncomp_size = prm->conncomp_size;
-    std::vector<HostPlan> prow(n), pcol(n);
+    std::vector<HostPlan> prow(n);
     for (int gi = 0; gi < n; gi++) {
         const int g = idx[gi];
         const unw_grid& q = grids[g];
@@ -659,85 +601,53 @@ int prepare(Solver& S, const std::vector<int>& idx, const unw_grid* grids, const
         G.ntiles = (int)(((long long)G.H * G.W + 4095) / 4096);
         if (G.H == 0) continue;
         prow[gi] = make_plan(G.W);
-        pcol[gi] = make_plan(G.H);
-        const HostPlan* pl[2] = {&prow[gi], &pcol[gi]};
-        DctPlanDev* dp[2] = {&G.prow, &G.pcol};
-        size_t tw[2] = {L.tw_r, L.tw_c}, hs[2] = {L.hs_r, L.hs_c}, dw[2] = {L.dw_r, L.dw_c},
-               ch[2] = {L.ch_r, L.ch_c};
-        int capn[2] = {L.fr_cap, L.fc_cap};
-        for (int d = 0; d < 2; d++) {
-            const HostPlan& hp = *pl[d];
-            if (hp.n > MAX_GEN || hp.n > capn[d] || (int)hp.rad.size() > UNW_MAX_PASSES)
-                return set_err(UNW_E_UNSUPPORTED, "grid %d: transform length %d (from %d) exceeds %d", g, hp.n,
-                               hp.N, MAX_GEN);
-            DctPlanDev& D = *dp[d];
-            D.N = hp.N;
-            D.blue = hp.blue;
-            D.stride = hp.n;
-            D.fft.n = hp.n;
-            D.fft.npass = (int)hp.rad.size();
-            for (size_t i = 0; i < hp.rad.size(); i++) D.fft.radix[i] = hp.rad[i];
-            D.fft.tw = (const float2*)(gb + tw[d]);
-            D.dctw = (const float2*)(gb + dw[d]);
-            D.chirp = (const float2*)(gb + ch[d]);
-            D.hspec = (const float2*)(gb + hs[d]);
-        }
+        const HostPlan& hp = prow[gi];
+        const HostPlan hc = make_plan(G.H);
+        // the column pass has no transform, but the supported sizes are those of the transforms
+        for (const HostPlan* q2 : {&hp, &hc})
+            if (q2->n > MAX_GEN || (int)q2->rad.size() > UNW_MAX_PASSES)
+                return set_err(UNW_E_UNSUPPORTED, "grid %d: transform length %d (from %d) exceeds %d", g, q2->n,
+                               q2->N, MAX_GEN);
+        if (hp.n > L.fr_cap)
+            return set_err(UNW_E_UNSUPPORTED, "grid %d: transform length %d (from %d) exceeds %d", g, hp.n, hp.N,
+                           L.fr_cap);
+        DctPlanDev& D = G.prow;
+        D.N = hp.N;
+        D.blue = hp.blue;
+        D.stride = hp.n;
+        D.fft.n = hp.n;
+        D.fft.npass = (int)hp.rad.size();
+        for (size_t i = 0; i < hp.rad.size(); i++) D.fft.radix[i] = hp.rad[i];
+        D.fft.tw = (const float2*)(gb + L.tw_r);
+        D.dctw = (const float2*)(gb + L.dw_r);
+        D.chirp = (const float2*)(gb + L.ch_r);
+        D.hspec = (const float2*)(gb + L.hs_r);
         // row kernel: one complex sequence (two rows) of fft_len(W)
-        const int rT = pick_threads(prow[gi].n, prow[gi].cap);
-        // column kernel: nseq column pairs of fft_len(H) under the shared-memory budget
-        int nseq = col_nseq_generic(pcol[gi].n, G.W);
-        int cT = 0;
-        while (nseq >= 1 && !(cT = pick_threads((long long)nseq * pcol[gi].n, pcol[gi].cap))) nseq--;
-        if (!rT || !cT) return set_err(UNW_E_UNSUPPORTED, "grid %d: no launch shape", g);
-        G.col_nseq = nseq;
+        const int rT = pick_threads(hp.n, hp.cap);
+        if (!rT) return set_err(UNW_E_UNSUPPORTED, "grid %d: no launch shape", g);
         S.sh.row_T = std::max(S.sh.row_T, rT);
-        S.sh.col_T = std::max(S.sh.col_T, cT);
-        S.sh.row_emax = std::max(S.sh.row_emax, prow[gi].emax);
-        S.sh.col_emax = std::max(S.sh.col_emax, pcol[gi].emax);
-        S.sh.row_smem = std::max(S.sh.row_smem, (size_t)prow[gi].n * sizeof(float2));
-        S.sh.col_smem = std::max(S.sh.col_smem, (size_t)nseq * pcol[gi].n * sizeof(float2));
+        S.sh.row_emax = std::max(S.sh.row_emax, hp.emax);
+        S.sh.row_smem = std::max(S.sh.row_smem, (size_t)hp.n * sizeof(float2));
+        G.tri = (const double*)(gb + L.tri);
+        S.sh.tri_L = unw_tri_rows(G.H, G.W);  // one value per launch group (group_key)
+        G.col_ctas = unw_tri_shape(G.H, G.W, S.sh.tri_L, &G.tri_ws, &G.tri_as, &G.tri_nta, &G.tri_ntb);
+        G.Tz = G.p1;
         G.sten_tiles_x = (G.W + 127) / 128;
         G.sten_rows = 1;
     }
-    // power-of-two register-FFT paths when every grid shares the dimension
+    // power-of-two or Bluestein register-FFT row passes when every grid has the length
     {
-        int w = -1, h = -1;
-        bool wsame = true, hsame = true;
+        int w = -1, mw = -1;
+        bool wsame = true, mwsame = true;
         for (int g = 0; g < n; g++) {
             const GridDev& G = S.hg[g];
             if (G.H == 0) continue;
+            const int a = bl_len(G.W);
             if (w < 0) w = G.W; else wsame &= (w == G.W);
-            if (h < 0) h = G.H; else hsame &= (h == G.H);
+            if (mw < 0) mw = a; else mwsame &= (mw == a);
         }
         if (w > 0 && wsame && unw_p2_col_nseq(w) > 0 && (w & (w - 1)) == 0) S.sh.row_p2 = w;
-        if (h > 0 && hsame && unw_p2_col_nseq(h) > 0 && (h & (h - 1)) == 0) {
-            S.sh.col_p2 = h;
-            for (int g = 0; g < n; g++) S.hg[g].col_nseq = unw_p2_col_nseq(h);
-        }
-        // Bluestein register-FFT paths when every grid has the same M along the axis
-        int mw = -1, mh = -1;
-        bool mwsame = true, mhsame = true;
-        for (int g = 0; g < n; g++) {
-            const GridDev& G = S.hg[g];
-            if (G.H == 0) continue;
-            const int a = bl_len(G.W), b = bl_len(G.H);
-            if (mw < 0) mw = a; else mwsame &= (mw == a);
-            if (mh < 0) mh = b; else mhsame &= (mh == b);
-        }
         if (!S.sh.row_p2 && mw > 0 && mwsame) S.sh.row_bl = mw;
-        if (!S.sh.col_p2 && mh > 0 && mhsame) {
-            S.sh.col_bl = mh;
-            for (int g = 0; g < n; g++) S.hg[g].col_nseq = unw_bl_col_nseq(mh);
-        }
-        // persistent column pass: 148 x min(4, 2048 / threads) CTAs.  This is more than the
-        // register limit lets reside at once (2 per SM at 512 threads), so a second wave starts
-        // as first-wave CTAs finish; measured at 4096^2 that beats sizing the grid to the
-        // resident count (102 us vs 113 us per launch), as the late CTAs fill the tail
-        const int cthreads = S.sh.col_p2 ? S.sh.col_p2 / 16 * unw_p2_col_nseq(S.sh.col_p2)
-                             : S.sh.col_bl ? S.sh.col_bl / 16 * unw_bl_col_nseq(S.sh.col_bl)
-                                           : S.sh.col_T;
-        const int per_sm = std::max(1, std::min(4, 2048 / std::max(cthreads, 1)));
-        for (int g = 0; g < n; g++) S.hg[g].col_ctas = NUM_SMS * per_sm;
     }
     // tensor-core column pass (mixed precision): every grid of the group has the same
     // H <= UNW_TC_MAX_H (one pair of DCT matrices for the launch)
@@ -776,9 +686,10 @@ int prepare(Solver& S, const std::vector<int>& idx, const unw_grid* grids, const
         GridDev& G = S.hg[g];
         if (G.H == 0) continue;
         CK(unw_launch_tables(G.prow.fft, G.prow, const_cast<float*>(G.sW), G.W, s));
-        CK(unw_launch_tables(G.pcol.fft, G.pcol, const_cast<float*>(G.sH), G.H, s));
         if (G.prow.blue) CK(unw_launch_hspec(pick_threads(prow[g].n, prow[g].cap), prow[g].emax, G.prow, s));
-        if (G.pcol.blue) CK(unw_launch_hspec(pick_threads(pcol[g].n, pcol[g].cap), pcol[g].emax, G.pcol, s));
+        CK(unw_tri_tables(const_cast<double*>(G.tri), G.H, G.W, s));
+        // column eigenvalue parts of the tensor-core pass (no transform tables: empty plan)
+        if (tc_h > 0) CK(unw_launch_tables(FftPlanDev{}, DctPlanDev{}, const_cast<float*>(G.sH), G.H, s));
         CK(cudaMemsetAsync(G.hist, 0, sizeof(int) * HIST_CAP, s));
     }
     if (tc_h > 0) {
@@ -807,29 +718,27 @@ int prepare(Solver& S, const std::vector<int>& idx, const unw_grid* grids, const
         }
         cudaGetLastError();
     }
-    // power-of-two column pass with the slab moved by TMA: per-grid tensor maps of T (even and
-    // odd rows) in the grid's 256-byte map slot (the tensor-core pass, which uses the same slots,
-    // covers H <= 1024 only)
-    S.sh.col_p2_tma = 0;
-    if (!S.sh.col_tc && S.sh.col_p2 && unw_p2_tma_nseq(S.sh.col_p2) > 0 && !(prm->flags & UNW_F_COL_NO_TMA)) {
+    if (S.sh.col_tc) {  // the tensor-core pass works in place on T
+        for (int g = 0; g < n; g++) S.hg[g].Tz = S.hg[g].T;
+        CK(cudaMemcpyAsync(S.dg, S.hg.data(), sizeof(GridDev) * n, cudaMemcpyHostToDevice, s));
+    }
+    // column pass with its tiles moved by TMA, on request only: the plain loads keep two CTAs per
+    // SM where a 128 KB tile leaves room for one (4096 x 4096: 45.5 us per launch, TMA 59.4; 1024 x 1024:
+    // 12.9 / 14.4).  The tensor map of T sits in the grid's map slot, which the tensor-core pass
+    // uses too.
+    S.sh.tri_tma = 0;
+    if (!S.sh.col_tc && S.sh.tri_L > 0 && (prm->flags & UNW_F_COL_TMA) && !(prm->flags & UNW_F_COL_NO_TMA)) {
         unsigned char* h = S.host_maps(n);
         bool ok = true;
         for (int g = 0; g < n && ok; g++) {
             const GridDev& G = S.hg[g];
             if (G.H > 0)
-                ok = G.col_nseq == unw_p2_tma_nseq(S.sh.col_p2) &&
-                     unw_p2_tma_maps(G.T, G.H, G.W, G.P, G.col_nseq,
-                                     h + UNW_MAP_BYTES * (size_t)g + 128 * UNW_MAP_COL);
+                ok = unw_tri_map(G.T, G.H, G.W, G.P, h + UNW_MAP_BYTES * (size_t)g + 128 * UNW_MAP_COL);
         }
         if (ok) {
             S.bmaps = base + B.tcmaps + UNW_MAP_BYTES * (size_t)slot;
             CK(cudaMemcpyAsync(S.bmaps, h, UNW_MAP_BYTES * (size_t)n, cudaMemcpyHostToDevice, s));
-            S.sh.col_p2_tma = 1;
-            if (!(prm->flags & UNW_F_COL_TMA)) {
-                int Wsum = 0;
-                for (int g = 0; g < n; g++) Wsum += S.hg[g].W;
-                S.sh.col_p2_tma = autotune_tma(S, S.sh.col_p2, Wsum);
-            }
+            S.sh.tri_tma = 1;
         }
     }
     // matvec on TMA-staged halo tiles: per-grid maps of p, wIx and wIy in the grid's map slot
@@ -879,6 +788,11 @@ int solve_group(const std::vector<int>& idx, const unw_grid* grids, const std::v
         PL(UNW_PROF_ROW_RHO, L_rowf(S, 0, 0, 0));
         PL(UNW_PROF_COL, L_col(S, 0));
         PL(UNW_PROF_ROW_INV, L_rowi(S, 0));
+        // one refinement of the initial solution (float64 residual): the first IRLS weights, and
+        // through them the whole iteration, see u0 without the rounding of the float32 transforms
+        PL(UNW_PROF_ROW_RHO, L_rowf(S, 5, 0, 0));
+        PL(UNW_PROF_COL, L_col(S, 0));
+        PL(UNW_PROF_ROW_INV, L_rowi(S, 4));
         PL(UNW_PROF_ELEM, unw_launch_simple(UNW_K_INIT_RECENTRE, S.total[KS_ELEM], s, S.dg, S.ds(KS_ELEM), n, 0, S.sc));
 
         // 5. IRLS loop (utils_unwrap2d.py:1533-1626)
@@ -983,7 +897,7 @@ int solve_group(const std::vector<int>& idx, const unw_grid* grids, const std::v
             o.k_median = st.kmed;
             for (int i = 0; i < 64 && i < UNW_MAX_LOG; i++) o.cg_iters[i] = G.H ? st.cg_log[i] : 0;
             o.col_path = S.sh.col_tc;
-            o.col_tma = S.sh.col_p2_tma;
+            o.col_tma = S.sh.tri_tma;
             o.tune_ms[0] = S.tune.ms_fft;
             o.tune_ms[1] = S.tune.ms_tc;
             o.resid_rel = st.resid_rel;
@@ -1043,7 +957,7 @@ int solve_batch(int n, const unw_grid* grids, const unw_params* prm, void* ws, s
     // another on the caller's stream, so that the per-launch timings stay serial.
     std::map<std::array<int, 4>, std::vector<int>> groups;
     for (int g = 0; g < n; g++)
-        groups[group_key(bbox[4 * g + 1] - bbox[4 * g], bbox[4 * g + 3] - bbox[4 * g + 2])].push_back(g);
+        groups[group_key(bbox[4 * g + 1] - bbox[4 * g], bbox[4 * g + 3] - bbox[4 * g + 2], prm->flags)].push_back(g);
     if (stats)
         for (int g = 0; g < n; g++) memset(&stats[g], 0, sizeof(unw_stats));
     struct Job {
@@ -1177,7 +1091,7 @@ int adjoint_group(const std::vector<int>& idx, const unw_adj_grid* grids, const 
         CK(unw_launch_adj(UNW_A_REFINE, ne, s, S.dg, S.ds(KS_ELEM), n, 0));
         if (k == UNW_ADJ_REFINE) break;
         CK(unw_launch_adj(UNW_A_REFINE, ne, s, S.dg, S.ds(KS_ELEM), n, 1));
-        CK(L_rowf(S, 1, 1, 0));
+        CK(L_rowf(S, 4, 1, 0));
         CK(L_col(S, 1));
         CK(L_rowi(S, 1));
         rc = pcg_chunked(S, 1, UNW_ADJ_CHUNK);
@@ -1201,7 +1115,7 @@ int adjoint_group(const std::vector<int>& idx, const unw_adj_grid* grids, const 
     CK(unw_launch_adj(UNW_A_LSUM, ne, s, S.dg, S.ds(KS_ELEM), n));
     CK(unw_launch_adj(UNW_A_RHS, ne, s, S.dg, S.ds(KS_ELEM), n));
     CK(unw_launch_adj(UNW_A_REARM, 1, s, S.dg, nullptr, n));
-    CK(L_rowf(S, 1, 1, 0));
+    CK(L_rowf(S, 4, 1, 0));
     CK(L_col(S, 1));
     CK(L_rowi(S, 1));
     rc = pcg_chunked(S, 1, UNW_ADJ_CHUNK);
@@ -1302,7 +1216,7 @@ int adjoint_batch(int n, const unw_adj_grid* grids, const unw_params* prm, void*
     std::map<std::array<int, 4>, std::vector<int>> groups;
     for (int g = 0; g < n; g++) {
         const int h = bbox[4 * g + 1] - bbox[4 * g], w = bbox[4 * g + 3] - bbox[4 * g + 2];
-        if (h > 0 && w > 0) groups[group_key(h, w)].push_back(g);
+        if (h > 0 && w > 0) groups[group_key(h, w, 0)].push_back(g);
     }
     int ret = UNW_OK, slot = 0, soff = 0;
     for (auto& kv : groups) {

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL::T, MODE>())) k_rowf
             if (has1) Tb[k] = w.x * Vb.x - w.y * Vb.y;
         }
     }
-    if (MODE == 0 || MODE == 3) return;
+    if (MODE == 0 || MODE == 3 || MODE == 5) return;
     if (arrive<2>(G, local, nct, acc, red)) {
         finish_sum<2>(G, nct, acc, red);
         if (threadIdx.x == 0) rowfwd_finalize<MODE>(st, acc);
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const
     for (int pair = local; pair < (H + 1) / 2; pair += nct) {
         const int i0 = 2 * pair, i1 = i0 + 1;
         const bool has1 = i1 < H;
-        const float* __restrict__ Ta = G.T + (size_t)i0 * P;
-        const float* __restrict__ Tb = G.T + (size_t)i1 * P;
+        const float* __restrict__ Ta = G.Tz + (size_t)i0 * P;
+        const float* __restrict__ Tb = G.Tz + (size_t)i1 * P;
         __syncthreads();  // previous row pair's reads of sm are done
         // DCT-III pre-twiddle: V'_k = conj(w_k) (Y_k - i Y_{W-k}), Y_W = 0; store conj(C')
         for (int k = t; k < W; k += T) {
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const
             }
         }
     }
-    if (MODE != 0) return;
+    if (MODE != 0 && MODE != 4) return;
     if (arrive<2>(G, local, nct, acc, red)) {
         finish_sum<2>(G, nct, acc, red);
         if (threadIdx.x == 0) rowinv_finalize_initu(st, acc);
@@ -203,6 +203,8 @@ cudaError_t rowf_bl_m(int mode, int nblk, cudaStream_t s, const GridDev* gd, con
         case 0: return go(k_rowf_bl<BL, 0>);
         case 1: return go(k_rowf_bl<BL, 1>);
         case 2: return go(k_rowf_bl<BL, 2>);
+        case 4: return go(k_rowf_bl<BL, 4>);
+        case 5: return go(k_rowf_bl<BL, 5>);
         default: return go(k_rowf_bl<BL, 3>);
     }
 }
@@ -219,6 +221,7 @@ cudaError_t rowi_bl_m(int mode, int nblk, cudaStream_t s, const GridDev* gd, con
         case 0: return go(k_rowi_bl<BL, 0>);
         case 1: return go(k_rowi_bl<BL, 1>);
         case 2: return go(k_rowi_bl<BL, 2>);
+        case 4: return go(k_rowi_bl<BL, 4>);
         default: return go(k_rowi_bl<BL, 3>);
     }
 }

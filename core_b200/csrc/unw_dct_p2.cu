@@ -7,9 +7,10 @@
 // n/2 for even n, N-1-(n-1)/2 for odd n) is a scatter into / gather from
 // shared memory, so it costs no extra pass over HBM.
 //
-// Column pass: NSEQ column pairs per CTA; forward FFT, spectral step on
-// frequency pairs (k, N-k) in shared memory (DCT-II extraction, -1/lambda
-// scaling, DCT-III pre-twiddle), inverse FFT, store.
+// Column pass (allocation-free preconditioner only; the solver's is unw_col_tri.cu):
+// NSEQ column pairs per CTA; forward FFT, spectral step on frequency pairs (k, N-k) in
+// shared memory (DCT-II extraction, -1/lambda scaling, DCT-III pre-twiddle), inverse FFT,
+// store.
 #include "unw_regfft.cuh"
 #include "unw_rowops.cuh"
 #include "unw_colspec.cuh"
@@ -51,30 +52,36 @@ __device__ __forceinline__ float4 rowf_vals4(const GridDev& G, float* __restrict
     } else if (MODE == 3) {
         return ld4f(G.r, o);
     } else if (MODE == 1) {
-        // r = b - A x0 at columns j..j+3, neighbour differences from the pair (rowfwd_value mode 1)
+        // r = b - A x0 at columns j..j+3 in divergence form (resid_at_pair)
         const int H = G.H, W = G.W, P = G.P;
-        const float4 x4 = ld4f(U, o), l4 = ld4f(Lo, o), b4 = ld4f(G.b, o), wx4 = ld4f(G.wIx, o), wy4 = ld4f(G.wIy, o);
+        const float4 x4 = ld4f(U, o), l4 = ld4f(Lo, o), wx4 = ld4f(G.wIx, o), wy4 = ld4f(G.wIy, o);
+        const float4 gx4 = ld4f(G.gx, o), gy4 = ld4f(G.gy, o);
         const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 xu4 = i > 0 ? ld4f(U, o - P) : z4, lu4 = i > 0 ? ld4f(Lo, o - P) : z4;
-        const float4 wyu4 = i > 0 ? ld4f(G.wIy, o - P) : z4;
+        const float4 wyu4 = i > 0 ? ld4f(G.wIy, o - P) : z4, gyu4 = i > 0 ? ld4f(G.gy, o - P) : z4;
         const float4 xd4 = i < H - 1 ? ld4f(U, o + P) : z4, ld4 = i < H - 1 ? ld4f(Lo, o + P) : z4;
         const float xl = j > 0 ? U[o - 1] : 0.f, ll = j > 0 ? Lo[o - 1] : 0.f;
-        const float wxl = j > 0 ? G.wIx[o - 1] : 0.f;
+        const float wxl = j > 0 ? G.wIx[o - 1] : 0.f, gxl = j > 0 ? G.gx[o - 1] : 0.f;
         const float xr = j + 4 < W ? U[o + 4] : 0.f, lr = j + 4 < W ? Lo[o + 4] : 0.f;
         const double xs[6] = {pair_val(xl, ll), pair_val(x4.x, l4.x), pair_val(x4.y, l4.y), pair_val(x4.z, l4.z),
                               pair_val(x4.w, l4.w), pair_val(xr, lr)};
         const float wxs[5] = {wxl, wx4.x, wx4.y, wx4.z, wx4.w};
+        const float gxs[5] = {gxl, gx4.x, gx4.y, gx4.z, gx4.w};
         float out[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const int jj = j + q;
             const double xc = xs[q + 1];
-            float res = 0.f;
-            if (jj > 0) res = fsub(res, fmul(dpair_diff(xc, xs[q]), wxs[q]));
-            if (jj < W - 1) res = fadd(res, fmul(dpair_diff(xs[q + 2], xc), wxs[q + 1]));
-            if (i > 0) res = fsub(res, fmul(dpair_diff(xc, pair_val(f4get(xu4, q), f4get(lu4, q))), f4get(wyu4, q)));
-            if (i < H - 1) res = fadd(res, fmul(dpair_diff(pair_val(f4get(xd4, q), f4get(ld4, q)), xc), f4get(wy4, q)));
-            const float val = fsub(f4get(b4, q), -res);
+            double r = 0.0;
+            if (jj > 0) r = fma((double)wxs[q], (double)gxs[q] - (xc - xs[q]), r);
+            if (jj < W - 1) r = fma(-(double)wxs[q + 1], (double)gxs[q + 1] - (xs[q + 2] - xc), r);
+            if (i > 0)
+                r = fma((double)f4get(wyu4, q),
+                        (double)f4get(gyu4, q) - (xc - pair_val(f4get(xu4, q), f4get(lu4, q))), r);
+            if (i < H - 1)
+                r = fma(-(double)f4get(wy4, q),
+                        (double)f4get(gy4, q) - (pair_val(f4get(xd4, q), f4get(ld4, q)) - xc), r);
+            const float val = (float)r;
             out[q] = val;
             acc[0] += isfinite(val) ? 0.0 : 1.0;
             acc[1] += (double)val * (double)val;
@@ -93,7 +100,7 @@ __device__ __forceinline__ float4 rowf_vals4(const GridDev& G, float* __restrict
     }
 }
 
-// The PCG-start pass (mode 1) forms b - A x0 from the iterate pair (eleven float4 rows
+// The PCG-start pass (mode 1) forms b - A x0 from the iterate pair (twelve float4 rows
 // in flight): it runs once per IRLS iteration and takes half the resident CTAs for the
 // registers that keep it from spilling.
 template <int T, int MODE>
@@ -169,7 +176,7 @@ __global__ void __launch_bounds__(N / 16, (rowf_blocks<N / 16, MODE>())) k_rowf_
         if (has1) st4f(Tb, 4 * c4, make_float4(xb[0], xb[1], xb[2], xb[3]));
     }
     }
-    if (MODE == 0 || MODE == 3) return;
+    if (MODE == 0 || MODE == 3 || MODE == 5) return;
     if (arrive<2>(G, local, nct, acc, red)) {
         finish_sum<2>(G, nct, acc, red);
         if (threadIdx.x == 0) rowfwd_finalize<MODE>(st, acc);
@@ -192,6 +199,11 @@ __device__ __forceinline__ void rowi_store4(const GridDev& G, int i, int j, floa
         const uchar4 v = *reinterpret_cast<const uchar4*>(G.valid + o);
         acc[0] += (double)(u.x * (v.x ? 1.f : 0.f)) + (double)(u.y * (v.y ? 1.f : 0.f)) +
                   (double)(u.z * (v.z ? 1.f : 0.f)) + (double)(u.w * (v.w ? 1.f : 0.f));
+    } else if (MODE == 4) {
+        rowinv_store<4>(G, i, j, z.x, beta, acc);
+        rowinv_store<4>(G, i, j + 1, z.y, beta, acc);
+        rowinv_store<4>(G, i, j + 2, z.z, beta, acc);
+        rowinv_store<4>(G, i, j + 3, z.w, beta, acc);
     } else if (MODE == 1) {
         st4f(G.p0, o, z);
     } else {
@@ -230,8 +242,8 @@ __global__ void __launch_bounds__(N / 16, min_blocks<N / 16>()) k_rowi_p2(const 
     for (int pair = local; pair < (H + 1) / 2; pair += nct) {
     const int i0 = 2 * pair, i1 = i0 + 1;
     const bool has1 = i1 < H;
-    const float* __restrict__ Ta = G.T + (size_t)i0 * P;
-    const float* __restrict__ Tb = G.T + (size_t)i1 * P;
+    const float* __restrict__ Ta = G.Tz + (size_t)i0 * P;
+    const float* __restrict__ Tb = G.Tz + (size_t)i1 * P;
     if (MODE == 2) {
         // the epilogue reads p of these rows after the FFT: start them towards L2 now
         const float* ra = G.p0 + (size_t)i0 * P;
@@ -374,25 +386,20 @@ __global__ void __launch_bounds__(N / 16, min_blocks<N / 16>()) k_rowi_p2(const 
         }
     }
     }
-    if (MODE != 0) return;
+    if (MODE != 0 && MODE != 4) return;
     if (arrive<2>(G, local, nct, acc, red)) {
         finish_sum<2>(G, nct, acc, red);
         if (threadIdx.x == 0) rowinv_finalize_initu(st, acc);
     }
 }
 
-// MODE 0: DCT initial solve (always runs); MODE 1 / 2: PCG (gated), also
-// r.z by Parseval and its scalar step (col_finalize).
-template <int N, int NSEQ, int MODE>
+template <int N, int NSEQ>
 __global__ void __launch_bounds__(N / 16 * NSEQ, min_blocks<N / 16 * NSEQ>()) k_col_p2(
     const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
     constexpr int T = N / 16;
     extern __shared__ float2 sm[];
-    __shared__ double red[32];
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
-    InstState* st = G.st;
-    if (MODE >= 1 && !(st->irls_active && st->cg_active)) return;
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const int W = G.W, P = G.P;
@@ -404,7 +411,6 @@ __global__ void __launch_bounds__(N / 16 * NSEQ, min_blocks<N / 16 * NSEQ>()) k_
     const float* __restrict__ sH = G.sH;
     const float negs = -1.0f / (4.0f * (float)N * (float)W);
     const int nslab = (W + 2 * NSEQ - 1) / (2 * NSEQ);
-    double acc[1] = {0.0};
     for (int slab = local; slab < nslab; slab += nct) {
     const int ja = 2 * NSEQ * slab + 2 * s;
     const bool hasa = ja < W, hasb = ja + 1 < W;
@@ -427,7 +433,7 @@ __global__ void __launch_bounds__(N / 16 * NSEQ, min_blocks<N / 16 * NSEQ>()) k_
     __syncthreads();  // previous slab's reads of sm are done
     io_fft<N, true, false>(v, sms, t, tw);
     const float ca = hasa ? G.sW[ja] : 1.0f, cb = hasb ? G.sW[ja + 1] : 1.0f;
-    col_spectral_p2<N, MODE>(sms, t, dw, sH, ca, cb, ja == 0, hasb, negs, acc[0]);
+    col_spectral_p2<N>(sms, t, dw, sH, ca, cb, ja == 0, hasb, negs);
     __syncthreads();
     io_fft<N, false, true>(v, sms, t, tw);
 #pragma unroll
@@ -437,11 +443,6 @@ __global__ void __launch_bounds__(N / 16 * NSEQ, min_blocks<N / 16 * NSEQ>()) k_
         else if (hasb) { a[0] = v[q].x; a[1] = -v[q].y; }
         else if (hasa) a[0] = v[q].x;
     }
-    }
-    if (MODE == 0) return;
-    if (arrive<1>(G, local, nct, acc, red)) {
-        finish_sum<1>(G, nct, acc, red);
-        if (threadIdx.x == 0) col_finalize<MODE>(st, acc[0]);
     }
 }
 
@@ -459,6 +460,8 @@ static cudaError_t rowf_p2_n(int mode, int nblk, cudaStream_t s, const GridDev* 
         case 0: return go(k_rowf_p2<N, 0>);
         case 1: return go(k_rowf_p2<N, 1>);
         case 2: return go(k_rowf_p2<N, 2>);
+        case 4: return go(k_rowf_p2<N, 4>);
+        case 5: return go(k_rowf_p2<N, 5>);
         default: return go(k_rowf_p2<N, 3>);
     }
 }
@@ -475,6 +478,7 @@ static cudaError_t rowi_p2_n(int mode, int nblk, cudaStream_t s, const GridDev* 
         case 0: return go(k_rowi_p2<N, 0>);
         case 1: return go(k_rowi_p2<N, 1>);
         case 2: return go(k_rowi_p2<N, 2>);
+        case 4: return go(k_rowi_p2<N, 4>);
         default: return go(k_rowi_p2<N, 3>);
     }
 }
@@ -495,19 +499,12 @@ constexpr int col_nseq_p2() {
 }
 
 template <int N>
-static cudaError_t col_p2_n(int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* st, int n) {
+static cudaError_t col_p2_n(int nblk, cudaStream_t s, const GridDev* gd, const int* st, int n) {
     constexpr int NS = col_nseq_p2<N>();
     const size_t smem = sizeof(float2) * RegFft<N>::SEQ_STRIDE * NS;
-    auto go = [&](auto kfn) {
-        cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kfn<<<nblk, N / 16 * NS, smem, s>>>(gd, st, n);
-        return cudaGetLastError();
-    };
-    switch (mode) {
-        case 0: return go(k_col_p2<N, NS, 0>);
-        case 1: return go(k_col_p2<N, NS, 1>);
-        default: return go(k_col_p2<N, NS, 2>);
-    }
+    cudaFuncSetAttribute(k_col_p2<N, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_col_p2<N, NS><<<nblk, N / 16 * NS, smem, s>>>(gd, st, n);
+    return cudaGetLastError();
 }
 
 int unw_p2_col_nseq(int N) {
@@ -551,10 +548,9 @@ cudaError_t unw_launch_rowi_p2(int N, int mode, int nblk, cudaStream_t s, const 
 #undef CALL
 }
 
-cudaError_t unw_launch_col_p2(int N, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
-                              int n) {
+cudaError_t unw_launch_col_p2(int N, int nblk, cudaStream_t s, const GridDev* gd, const int* starts, int n) {
     if (nblk <= 0) return cudaSuccess;
-#define CALL(NN) col_p2_n<NN>(mode, nblk, s, gd, starts, n)
+#define CALL(NN) col_p2_n<NN>(nblk, s, gd, starts, n)
     UNW_P2_SWITCH(N, CALL)
 #undef CALL
 }

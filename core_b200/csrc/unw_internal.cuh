@@ -87,12 +87,13 @@ struct GridDev {
     float* out_u;        long long out_u_pitch;   // full-grid origin
     uint16_t* out_cc;    long long out_cc_pitch;
     int congruent;
-    int col_nseq;               // complex sequences (column pairs) per column CTA
-    int col_ctas;               // CTA cap of the persistent column pass
+    int col_nseq;               // complex sequences (column pairs) per CTA of the FFT column pass
+    int col_ctas;               // CTAs of this grid in the column pass
     int sten_rows;              // rows per stencil CTA
     int sten_tiles_x;           // column tiles per stencil row strip
     float *gx, *gy, *wx, *wy;
     float *wIx, *wIy, *b, *r, *z, *p0, *p1, *Ap, *T;
+    float* Tz;                  // what the column pass leaves for the row-inverse pass (p1, or T in place)
     // The IRLS iterate u is a float32 pair U + L with U = fl32(u) and |L| <= ulp(U)/2
     // (about 48 significant bits): U0/L0 and U1/L1 ping-pong per IRLS iteration, Ub/Lb
     // hold the best iterate.  The PCG accumulates its correction x - x0 in D (float32,
@@ -106,6 +107,9 @@ struct GridDev {
     // (utils_unwrap2d.py:1284-1289) without its cancellation near k = j = 0.
     const float* sH;
     const float* sW;
+    const double* tri;          // tridiagonal column pass: per-column constants,
+    int tri_ws, tri_as;         // ... groups of 32 wide columns, strips with the long halo,
+    int tri_nta, tri_ntb;       // ... tiles per strip with the long / short halo
     DctPlanDev prow, pcol;
     InstState* st;
     double* part;               // reduction partials [max CTAs][UNW_NPART]

@@ -66,8 +66,7 @@ cudaError_t unw_launch_row_fwd(int mode, int T, int emax, int nblk, size_t smem,
                                const GridDev* gd, const int* starts, int n, int it, int cgk);
 cudaError_t unw_launch_row_inv(int mode, int T, int emax, int nblk, size_t smem, cudaStream_t s,
                                const GridDev* gd, const int* starts, int n);
-cudaError_t unw_launch_col(int mode, int T, int emax, int nblk, size_t smem, cudaStream_t s,
-                           const GridDev* gd, const int* starts, int n);
+cudaError_t unw_launch_col(int T, int nblk, size_t smem, cudaStream_t s, const GridDev* gd, const int* starts, int n);
 cudaError_t unw_launch_simple(int which, int nblk, cudaStream_t s, const GridDev* gd,
                               const int* starts, int n, int it, UnwScalars sc);
 
@@ -77,17 +76,13 @@ cudaError_t unw_launch_rowf_p2(int N, int mode, int nblk, cudaStream_t s, const 
                                int n, int it, int cgk);
 cudaError_t unw_launch_rowi_p2(int N, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
                                int n);
-cudaError_t unw_launch_col_p2(int N, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
-                              int n);
+cudaError_t unw_launch_col_p2(int N, int nblk, cudaStream_t s, const GridDev* gd, const int* starts, int n);
 
 // Bluestein-on-register-FFT DCT passes for other lengths (M = power of two >= 2N - 1)
-int unw_bl_col_nseq(int M);
 cudaError_t unw_launch_rowf_bl(int M, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
                                int n, int it, int cgk);
 cudaError_t unw_launch_rowi_bl(int M, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
                                int n);
-cudaError_t unw_launch_col_bl(int M, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
-                              int n);
 
 // tensor-core (tcgen05, split-precision bf16) column pass for grids of H <= UNW_TC_MAX_H rows
 #define UNW_TC_MAX_H 1024
@@ -129,8 +124,7 @@ cudaError_t unw_launch_post(int which, int nblk, cudaStream_t s, const GridDev* 
                             int n, const UnwScalars& sc, const GridDev* host_grids);
 
 // Per-grid tensor maps of the TMA-staged passes (one 128-byte CUtensorMap each): the
-// column pass's two (tensor-core T / p1, or power-of-two even / odd rows of T) at
-// UNW_MAP_COL, the matvec's three (p, wIx, wIy) at UNW_MAP_MV.
+// column pass's (tensor-core T / p1, or the tridiagonal pass's T) at UNW_MAP_COL, the matvec's three (p, wIx, wIy) at UNW_MAP_MV.
 #define UNW_MAPS_PER_GRID 8
 #define UNW_MAP_BYTES (128 * UNW_MAPS_PER_GRID)
 #define UNW_MAP_COL 0
@@ -139,11 +133,16 @@ bool unw_mv_tma_maps(const float* p, const float* wIx, const float* wIy, int H, 
 cudaError_t unw_launch_matvec_tma(int nblk, cudaStream_t s, const GridDev* gd, const int* starts, int n,
                                   const void* maps);
 
-// power-of-two column pass with the slab moved by TMA (unw_dct_p2_tma.cu), H = 2048 / 4096
-int unw_p2_tma_nseq(int N);
-bool unw_p2_tma_maps(const float* T, int H, int W, int P, int nseq, void* out);
-cudaError_t unw_launch_col_p2_tma(int N, int mode, int nblk, cudaStream_t s, const GridDev* gd, const int* starts,
-                                  int n, const void* maps);
+// column pass as a tridiagonal solve per column (unw_col_tri.cu): rows per segment of a grid
+// (one value per launch), the shape of its CTAs (returns their number), its per-column table,
+// the tensor map of T (H x W, pitch P) for the TMA-staged form (false: not available)
+int unw_tri_rows(int H, int W);
+int unw_tri_shape(int H, int W, int L, int* ws, int* as, int* nta, int* ntb);
+size_t unw_tri_table_bytes(long long W);
+cudaError_t unw_tri_tables(double* tab, int H, int W, cudaStream_t s);
+bool unw_tri_map(const float* T, int H, int W, int P, void* out);
+cudaError_t unw_launch_col_tri(int L, bool tma, int mode, int nblk, cudaStream_t s, const GridDev* gd,
+                               const int* starts, int n, const void* maps);
 
 // frozen-weight adjoint (KS_ELEM shapes except REARM)
 #define UNW_ADJ_REFINE 3    // refinement passes of u* (each stops early below 1e-13 residual)

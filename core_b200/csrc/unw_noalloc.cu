@@ -158,6 +158,7 @@ extern "C" int unw_apply_preconditioner_noalloc(const float* r, int64_t H, int64
     G.r = const_cast<float*>(r);
     G.z = z;
     G.T = (float*)(base + UNW_NOALLOC_HEADER);
+    G.Tz = G.T;  // the column pass works in place
     G.st = (InstState*)(base + o_state);
     G.counter = (unsigned*)(base + o_cnt);
     G.sW = (const float*)(base + o_sw);
@@ -192,10 +193,10 @@ extern "C" int unw_apply_preconditioner_noalloc(const float* r, int64_t H, int64
     const int cthreads = col_p2 ? col_p2 / 16 * G.col_nseq : cT;
     int per_sm = 2048 / cthreads;
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
-    G.col_ctas = 148 * per_sm;
+    const int col_ctas = 148 * per_sm;
     const int n_row = (G.H + 1) / 2 < 148 * 4 ? (G.H + 1) / 2 : 148 * 4;
     const int nslab = (G.W + 2 * G.col_nseq - 1) / (2 * G.col_nseq);
-    const int n_col = nslab < G.col_ctas ? nslab : G.col_ctas;
+    const int n_col = nslab < col_ctas ? nslab : col_ctas;
     int starts[2 * (KS_NKIND + 1)];
     memset(starts, 0, sizeof(starts));
     starts[2 * KS_ROWPAIR + 1] = n_row;
@@ -217,8 +218,8 @@ extern "C" int unw_apply_preconditioner_noalloc(const float* r, int64_t H, int64
     e = row_p2 ? unw_launch_rowf_p2(row_p2, 3, n_row, s, dG, dS + 2 * KS_ROWPAIR, 1, 0, 0)
                : unw_launch_row_fwd(3, rT, 16, n_row, row_smem, s, dG, dS + 2 * KS_ROWPAIR, 1, 0, 0);
     if (e == cudaSuccess)
-        e = col_p2 ? unw_launch_col_p2(col_p2, 0, n_col, s, dG, dS + 2 * KS_COL, 1)
-                   : unw_launch_col(0, cT, 16, n_col, col_smem, s, dG, dS + 2 * KS_COL, 1);
+        e = col_p2 ? unw_launch_col_p2(col_p2, n_col, s, dG, dS + 2 * KS_COL, 1)
+                   : unw_launch_col(cT, n_col, col_smem, s, dG, dS + 2 * KS_COL, 1);
     if (e == cudaSuccess)
         e = row_p2 ? unw_launch_rowi_p2(row_p2, 3, n_row, s, dG, dS + 2 * KS_ROWPAIR, 1)
                    : unw_launch_row_inv(3, rT, 16, n_row, row_smem, s, dG, dS + 2 * KS_ROWPAIR, 1);

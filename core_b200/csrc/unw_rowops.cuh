@@ -19,45 +19,43 @@ __device__ __forceinline__ float lap_at(const float* __restrict__ x, const float
     return -res;
 }
 
-// Difference a - b of two iterate values held as float32 pairs: exact in float64,
-// rounded once to float32.  (A float32 form, fl(fl(ah - bh) + fl(al - bl)), is within a
-// few ulps of the difference too; on the 4096^2 fault grid, whose IRLS stop test is
-// decided by rel_change within about 1% of tol at the 29th iteration, that form ended
-// after 29 iterations where the reference's FP64 run takes 30, and this one takes 30.)
-__device__ __forceinline__ float pair_diff(float ah, float al, float bh, float bl) {
-    return __double2float_rn(((double)ah - (double)bh) + ((double)al - (double)bl));
-}
-// The same from the pairs' float64 values (hi + lo is exact in float64, and so is each of
-// the two differences above; both forms round the exact difference once): each pixel's
-// pair is converted once and shared by the differences it takes part in.
+// Difference a - b of two iterate values (float32 pairs as float64 values: hi + lo is exact, and so
+// is the difference), rounded once to float32.
 __device__ __forceinline__ float dpair_diff(double a, double b) { return __double2float_rn(a - b); }
 
-// A x at (i, j) for the iterate x = U + L held as a float32 pair: the reference's op
-// order (lap_at), each neighbour difference formed from the pair by pair_diff.
-__device__ __forceinline__ float lap_at_pair(const float* __restrict__ U, const float* __restrict__ L,
-                                             const float* __restrict__ wx, const float* __restrict__ wy, int i, int j,
-                                             int H, int W, int P) {
+// b - A x at (i, j) in divergence form, sum over the pixel's edges of +-w_e (g_e - (D x)_e) in
+// float64 from the float32 weights and gradients, x the pair U + L
+// (utils_unwrap2d.py:1413-1419, :1576-1581).  Formed as the difference of b and A x in float32 the rounding of
+// b, about 1e-7 of the largest w g and white, entered the solution as a smooth error through
+// A^-1 and was its largest error wherever the iteration converges.
+__device__ __forceinline__ double resid_at_pair(const float* __restrict__ U, const float* __restrict__ L,
+                                                const float* __restrict__ wx, const float* __restrict__ wy,
+                                                const float* __restrict__ gx, const float* __restrict__ gy, int i,
+                                                int j, int H, int W, int P) {
     const size_t o = (size_t)i * P + j;
     const double xc = pair_val(U[o], L[o]);
-    float res = 0.f;
-    if (j > 0) res = fsub(res, fmul(dpair_diff(xc, pair_val(U[o - 1], L[o - 1])), wx[o - 1]));
-    if (j < W - 1) res = fadd(res, fmul(dpair_diff(pair_val(U[o + 1], L[o + 1]), xc), wx[o]));
-    if (i > 0) res = fsub(res, fmul(dpair_diff(xc, pair_val(U[o - P], L[o - P])), wy[o - P]));
-    if (i < H - 1) res = fadd(res, fmul(dpair_diff(pair_val(U[o + P], L[o + P]), xc), wy[o]));
-    return -res;
+    double r = 0.0;
+    if (j > 0) r = fma((double)wx[o - 1], (double)gx[o - 1] - (xc - pair_val(U[o - 1], L[o - 1])), r);
+    if (j < W - 1) r = fma(-(double)wx[o], (double)gx[o] - (pair_val(U[o + 1], L[o + 1]) - xc), r);
+    if (i > 0) r = fma((double)wy[o - P], (double)gy[o - P] - (xc - pair_val(U[o - P], L[o - P])), r);
+    if (i < H - 1) r = fma(-(double)wy[o], (double)gy[o] - (pair_val(U[o + P], L[o + P]) - xc), r);
+    return r;
 }
 
 // Row-forward modes:
 //  0 RHO  rho = -div(w g), the DCT initial solve (utils_unwrap2d.py:1478-1483)
-//  1 R0   r = b - A x0, PCG start (utils_unwrap2d.py:1413-1419), with the neighbour
-//         differences of x0 formed from the iterate pair; D (the PCG correction) = 0
+//  1 R0   r = b - A x0, PCG start (utils_unwrap2d.py:1413-1419), from the iterate pair
+//         (resid_at_pair); D (the PCG correction) = 0
 //  2 UPD  x += alpha p; r -= alpha Ap (utils_unwrap2d.py:1445-1459); x is the
 //         correction D = x - x0, added to the iterate pair at the IRLS tail
 //  3 COPY r as given (operator entry point)
+//  4 RHS  r = b as given, x0 = 0, PCG start; D = 0 (adjoint solves)
+//  5 RHO1 residual of the DCT initial solution u0 = U0, -div(w g - grad u0) in float64
 template <int MODE>
 __device__ __forceinline__ bool rowfwd_gate(const InstState* s) {
     if (MODE == 0 || MODE == 3) return true;
-    if (MODE == 1) return s->irls_active != 0;
+    if (MODE == 5) return !(s->status & 1);  // not after a non-finite initial solution
+    if (MODE == 1 || MODE == 4) return s->irls_active != 0;
     return s->irls_active != 0 && s->cg_active != 0;
 }
 
@@ -84,9 +82,17 @@ __device__ __forceinline__ float rowfwd_value(const GridDev& G, float* __restric
         return rr;
     } else if (MODE == 3) {
         return G.r[o];
-    } else if (MODE == 1) {
-        const float ax = lap_at_pair(U, Lo, G.wIx, G.wIy, i, j, H, W, P);
-        const float val = fsub(G.b[o], ax);
+    } else if (MODE == 5) {
+        const float* __restrict__ u = G.U0;
+        const double xc = (double)u[o];
+        double r = 0.0;
+        if (j > 0) r += (double)G.wx[o - 1] * (double)G.gx[o - 1] - (xc - (double)u[o - 1]);
+        if (j < W - 1) r -= (double)G.wx[o] * (double)G.gx[o] - ((double)u[o + 1] - xc);
+        if (i > 0) r += (double)G.wy[o - P] * (double)G.gy[o - P] - (xc - (double)u[o - P]);
+        if (i < H - 1) r -= (double)G.wy[o] * (double)G.gy[o] - ((double)u[o + P] - xc);
+        return (float)r;
+    } else if (MODE == 1 || MODE == 4) {
+        const float val = MODE == 4 ? G.b[o] : (float)resid_at_pair(U, Lo, G.wIx, G.wIy, G.gx, G.gy, i, j, H, W, P);
         G.r[o] = val;
         G.D[o] = 0.f;
         acc[0] += isfinite(val) ? 0.0 : 1.0;
@@ -105,7 +111,7 @@ __device__ __forceinline__ float rowfwd_value(const GridDev& G, float* __restric
 
 template <int MODE>
 __device__ __forceinline__ void rowfwd_finalize(InstState* st, const double (&acc)[2]) {
-    if (MODE == 1) {
+    if (MODE == 1 || MODE == 4) {
         // non-finite initial residual: CG returns x0 (utils_unwrap2d.py:1418-1419)
         st->cg_active = acc[0] == 0.0 ? 1 : 0;
         if (st->cg_rel > 0.f) st->cg_tol = (float)((double)st->cg_rel * sqrt(acc[1]));
@@ -135,11 +141,13 @@ __device__ __forceinline__ void matvec_finalize(InstState* st, double pAp) {
 //  1 P0    p = z = M^-1 r                     (utils_unwrap2d.py:1421-1424)
 //  2 P     p = z + beta p, z = M^-1 r         (utils_unwrap2d.py:1461-1473)
 //  3 COPY  z as computed (operator entry point)
+//  4 INIT1 u0 + z as a pair into (U0, L0) (one refinement of the initial solution), sum of u * valid
 // r.z and beta come from the column pass (Parseval, col_finalize), so modes 1
 // and 2 write p in place and never store z.
 template <int MODE>
 __device__ __forceinline__ bool rowinv_gate(const InstState* s) {
     if (MODE == 0 || MODE == 3) return true;
+    if (MODE == 4) return !(s->status & 1);
     return s->irls_active != 0 && s->cg_active != 0;
 }
 
@@ -155,6 +163,13 @@ __device__ __forceinline__ void rowinv_store(const GridDev& G, int i, int j, flo
         G.U0[o] = u;
         // (u * valid_float).sum(): an invalid pixel contributes u * 0
         acc[0] += (double)(u * (G.valid[o] ? 1.f : 0.f));
+    } else if (MODE == 4) {
+        const double u = (double)G.U0[o] + (double)zv;
+        float hi, lo;
+        split_pair(u, hi, lo);
+        G.U0[o] = hi;
+        G.L0[o] = lo;
+        if (G.valid[o]) acc[0] += u;
     } else if (MODE == 1) {
         G.p0[o] = zv;
     } else {
@@ -191,16 +206,9 @@ __device__ __forceinline__ void col_finalize(InstState* st, double rzn) {
 // (k, km = H-k): the DCT-II extraction and the eigenvalue scaling are shared,
 // only the DCT-III pre-twiddles differ.  For k = 0 (km = 0) or k = km the
 // second output equals the first and is not used.
-//
-// RZ adds this pair's share of r.z to `rz` by Parseval's identity for the
-// unnormalised DCT-II / DCT-III pair: with X the 2-D DCT-II of r and Y the
-// scaled spectrum that the DCT-III turns into z,
-//     r.z = sum_{k,l} e_k e_l X_kl Y_kl,   e_0 = 1/2, e_{k>0} = 1,
-// so the preconditioned inner product needs no extra pass over r and z.
-template <bool RZ>
 __device__ __forceinline__ void col_spectral_pair(float2 C, float2 Cm, int k, int km, float2 wk, float2 wm,
                                                   float ck, float cm, float ca, float cb, bool ja0, bool hasb,
-                                                  float negs, float2& ok, float2& om, double& rz) {
+                                                  float negs, float2& ok, float2& om) {
     const float2 Vak = make_float2(C.x + Cm.x, C.y - Cm.y);
     const float2 Vbk = make_float2(C.y + Cm.y, Cm.x - C.x);
     const float2 Vam = make_float2(Vak.x, -Vak.y);   // conj: the pair's extraction is symmetric
@@ -213,13 +221,6 @@ __device__ __forceinline__ void col_spectral_pair(float2 C, float2 Cm, int k, in
     const float Xam = (km == 0 && ja0) ? 0.f : xam * __fdividef(negs, -(cm + ca));
     const float Xbk = hasb ? xbk * __fdividef(negs, -(ck + cb)) : 0.f;
     const float Xbm = hasb ? xbm * __fdividef(negs, -(cm + cb)) : 0.f;
-    if (RZ) {
-        const float ea = ja0 ? 0.5f : 1.0f;
-        float tk = fmaf(xak * ea, Xak, xbk * Xbk);
-        if (k == 0) tk *= 0.5f;
-        const float tm = km != k ? fmaf(xam * ea, Xam, xbm * Xbm) : 0.f;
-        rz += (double)tk + (double)tm;
-    }
     // DCT-III pre-twiddle V'_k = conj(w_k) (Y_k - i Y_{H-k}) with Y_H = 0
     const float mak = k == 0 ? 0.f : Xam, mbk = k == 0 ? 0.f : Xbm;
     const float2 Pak = cmul(cconj(wk), make_float2(Xak, -mak));

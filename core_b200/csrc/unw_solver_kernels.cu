@@ -10,7 +10,7 @@
 //
 // The DCT preconditioner (utils_unwrap2d.py:1390-1403) is three passes:
 //   row_fwd: row DCT-II of a pair of rows through one complex FFT,
-//   col:     column DCT-II -> scale by -1/lambda -> column DCT-III (fused),
+//   col:     a tridiagonal solve per column (unw_col_tri.cu),
 //   row_inv: row DCT-III of a pair of rows through one complex FFT,
 // each pass fused with the elementwise PCG work that reads or writes the
 // same rows.  Float32 elementwise arithmetic follows the reference's
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(T) k_row_fwd(const GridDev* __restrict__ grids
         if (has1) G.T[(size_t)i1 * P + k] = w.x * Vb.x - w.y * Vb.y;
     }
     }
-    if (MODE == 0 || MODE == 3) return;
+    if (MODE == 0 || MODE == 3 || MODE == 5) return;
     if (arrive<2>(G, local, nct, acc, red)) {
         finish_sum<2>(G, nct, acc, red);
         if (threadIdx.x == 0) rowfwd_finalize<MODE>(st, acc);
@@ -194,23 +194,19 @@ __global__ void __launch_bounds__(T) k_row_fwd(const GridDev* __restrict__ grids
 }
 
 // ============================================================ column pass
-// Column DCT-II -> scale by -1/(4 H W lambda) -> column DCT-III, in place on T.
-// MODE 0: DCT initial solve (always runs); MODE 1 / 2: PCG (gated), also
-// r.z by Parseval and its scalar step (col_finalize).
-template <int T, int EMAX, int MODE>
+// Column DCT-II -> scale by -1/(4 H W lambda) -> column DCT-III, in place on T, for the
+// allocation-free preconditioner (whose scratch has no room for the tridiagonal pass's table).
+template <int T>
 __global__ void __launch_bounds__(T) k_col(const GridDev* __restrict__ grids,
                                            const int* __restrict__ starts, int n) {
+    constexpr int EMAX = 16;
     extern __shared__ float2 sm[];
-    __shared__ double red[32];
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
-    InstState* st = G.st;
-    if (MODE >= 1 && !(st->irls_active && st->cg_active)) return;
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const int H = G.H, W = G.W, P = G.P;
     const int nslab = (W + 2 * G.col_nseq - 1) / (2 * G.col_nseq);
-    double acc[1] = {0.0};
     for (int slab = local; slab < nslab; slab += nct) {
     const int c0 = 2 * G.col_nseq * slab;
     const int nseq = min(G.col_nseq, (W - c0 + 1) >> 1);
@@ -243,8 +239,7 @@ __global__ void __launch_bounds__(T) k_col(const GridDev* __restrict__ grids,
         const float ca = sW[ja], cb = hasb ? sW[ja + 1] : 1.0f;
         const float2 wk = __ldg(&dw[k]), wm = __ldg(&dw[km]);
         float2 ok, om;
-        col_spectral_pair<(MODE >= 1)>(C, Cm, k, km, wk, wm, sH[k], sH[km], ca, cb, ja == 0, hasb, negs, ok, om,
-                                     acc[0]);
+        col_spectral_pair(C, Cm, k, km, wk, wm, sH[k], sH[km], ca, cb, ja == 0, hasb, negs, ok, om);
         if (km != k) base[km] = om;
         base[k] = ok;
     }
@@ -257,11 +252,6 @@ __global__ void __launch_bounds__(T) k_col(const GridDev* __restrict__ grids,
         Tm[(size_t)i * P + c] = v.x;
         if (c + 1 < W) Tm[(size_t)i * P + c + 1] = -v.y;
     }
-    }
-    if (MODE == 0) return;
-    if (arrive<1>(G, local, nct, acc, red)) {
-        finish_sum<1>(G, nct, acc, red);
-        if (threadIdx.x == 0) col_finalize<MODE>(st, acc[0]);
     }
 }
 
@@ -287,8 +277,8 @@ __global__ void __launch_bounds__(T) k_row_inv(const GridDev* __restrict__ grids
     const bool has1 = i1 < H;
     __syncthreads();  // previous row pair's reads of sm are done
     for (int k = threadIdx.x; k < W; k += T) {
-        const float a = G.T[(size_t)i0 * P + k];
-        const float b = has1 ? G.T[(size_t)i1 * P + k] : 0.f;
+        const float a = G.Tz[(size_t)i0 * P + k];
+        const float b = has1 ? G.Tz[(size_t)i1 * P + k] : 0.f;
         sm[k] = make_float2(a, b);
     }
     __syncthreads();
@@ -318,7 +308,7 @@ __global__ void __launch_bounds__(T) k_row_inv(const GridDev* __restrict__ grids
         if (has1) rowinv_store<MODE>(G, i1, j, -v.y, beta, acc);
     }
     }
-    if (MODE != 0) return;
+    if (MODE != 0 && MODE != 4) return;
     if (arrive<2>(G, local, nct, acc, red)) {
         finish_sum<2>(G, nct, acc, red);
         if (threadIdx.x == 0) rowinv_finalize_initu(st, acc);
@@ -434,16 +424,13 @@ __global__ void __launch_bounds__(512, 2) k_matvec(const GridDev* __restrict__ g
     }
 }
 
-// IRLS head (utils_unwrap2d.py:1536-1581): recentre, residual gradients,
-// best-iterate test, IRLS weights and right-hand side.  Reads the iterate pair
-// (U_cur, L_cur), writes the recentred pair to (U_nxt, L_nxt) (the current pair
-// keeps u_prev for the convergence test).  The residual gradients take the
-// neighbour differences of the pair (pair_diff; the mean cancels in them), the
-// recentred pair is formed in float64, the weights and b are float32 in the
-// reference's op order.
-// One warp per row, 4 columns per lane; the weight of the left edge comes from
-// the neighbouring lane, the weight of the upper edge is recomputed from the
-// row above (the same operations, so it equals that row's own value).
+// IRLS head (utils_unwrap2d.py:1536-1574): recentre, residual gradients, best-iterate test and
+// IRLS weights.  Reads the iterate pair (U_cur, L_cur), writes the recentred pair to
+// (U_nxt, L_nxt) (the current pair keeps u_prev for the convergence test).  The residual
+// gradients take the neighbour differences of the pair (the mean cancels in them), the
+// recentred pair is formed in float64, the weights are float32 in the reference's op order.
+// The right-hand side (:1576-1581) is not stored: the PCG start forms b - A x0 edge by edge.
+// One warp per row, 4 columns per lane.
 __device__ __forceinline__ float irls_w(float w, float r, float eps2) {
     return clampf_nan(fdiv(w, __fsqrt_rn(fadd(fmul(r, r), eps2))), 1e-6f, 1e6f);
 }
@@ -476,24 +463,22 @@ __global__ void __launch_bounds__(256, 4) k_head(const GridDev* __restrict__ gri
     const int j0 = tx * 128 + lane * 4;
     const int i = ty * 8 + warp;
     const bool on = i < H && j0 < W;
-    const bool hu = i > 0, hd = i < H - 1;
+    const bool hd = i < H - 1;
     const size_t o = (size_t)i * P + j0;
-    F4 u{}, l{}, ud{}, ld{}, uu{}, lu{}, gx{}, gy{}, gyu{}, wx{}, wy{}, wyu{};
-    float ul = 0.f, ll = 0.f, ur = 0.f, lr = 0.f, gxl = 0.f, wxl = 0.f;
+    F4 u{}, l{}, ud{}, ld{}, gx{}, gy{}, wx{}, wy{};
+    float ur = 0.f, lr = 0.f;
     if (on) {
         u = ld4(uc, o);
         l = ld4(lc, o);
         if (hd) { ud = ld4(uc, o + P); ld = ld4(lc, o + P); }
-        if (hu) { uu = ld4(uc, o - P); lu = ld4(lc, o - P); gyu = ld4(G.gy, o - P); wyu = ld4(G.wy, o - P); }
         gx = ld4(G.gx, o);
         gy = ld4(G.gy, o);
         wx = ld4(G.wx, o);
         wy = ld4(G.wy, o);
-        if (lane == 0 && j0 > 0) { ul = uc[o - 1]; ll = lc[o - 1]; gxl = G.gx[o - 1]; wxl = G.wx[o - 1]; }
         if (lane == 31 && j0 + 4 < W) { ur = uc[o + 4]; lr = lc[o + 4]; }
     }
     float rx[4], ry[4];
-    F4 wix, wiy, bv;
+    F4 wix, wiy;
     // the centre row's pairs as float64 values, converted once and shared (dpair_diff)
     double xv[4];
 #pragma unroll
@@ -511,30 +496,6 @@ __global__ void __launch_bounds__(256, 4) k_head(const GridDev* __restrict__ gri
         wix.v[q] = irls_w(wx.v[q], rx[q], eps2);
         wiy.v[q] = irls_w(wy.v[q], ry[q], eps2);
     }
-    float wl = __shfl_up_sync(0xffffffffu, wix.v[3], 1);
-    float gl = __shfl_up_sync(0xffffffffu, gx.v[3], 1);
-    if (lane == 0 && j0 > 0) {
-        const float rxl = fsub(dpair_diff(xv[0], pair_val(ul, ll)), gxl);
-        wl = irls_w(wxl, rxl, eps2);
-        gl = gxl;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int j = j0 + q;
-        float b = 0.f;
-        if (j > 0) {
-            const float wleft = q == 0 ? wl : wix.v[q - 1];
-            const float gleft = q == 0 ? gl : gx.v[q - 1];
-            b = fadd(b, fmul(wleft, gleft));
-        }
-        if (j < W - 1) b = fsub(b, fmul(wix.v[q], gx.v[q]));
-        if (hu) {
-            const float ryu = fsub(dpair_diff(xv[q], pair_val(uu.v[q], lu.v[q])), gyu.v[q]);
-            b = fadd(b, fmul(irls_w(wyu.v[q], ryu, eps2), gyu.v[q]));
-        }
-        if (hd) b = fsub(b, fmul(wiy.v[q], gy.v[q]));
-        bv.v[q] = b;
-    }
     if (on) {
         F4 ch, cl4;
 #pragma unroll
@@ -550,7 +511,6 @@ __global__ void __launch_bounds__(256, 4) k_head(const GridDev* __restrict__ gri
         st4(ln, o, cl4);
         st4(G.wIx, o, wix);
         st4(G.wIy, o, wiy);
-        st4(G.b, o, bv);
     }
     }
     if (arrive<2>(G, local, nct, acc, red)) {
@@ -612,12 +572,14 @@ __global__ void k_init_recentre(const GridDev* __restrict__ grids, const int* __
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const double m = st->vcount > 0 ? st->mean : 0.0;
+    const bool refined = !(st->status & 1);  // L0 is written unless the initial solution was non-finite
     UNW_ROWS_LOOP(G, local, nct) {
         const size_t o = (size_t)i * G.P + j;
         const F4 u = ld4(G.U0, o);
-        F4 hi, lo;
+        F4 l{}, hi, lo;
+        if (refined) l = ld4(G.L0, o);
 #pragma unroll
-        for (int q = 0; q < 4; q++) split_pair((double)u.v[q] - m, hi.v[q], lo.v[q]);
+        for (int q = 0; q < 4; q++) split_pair(pair_val(u.v[q], l.v[q]) - m, hi.v[q], lo.v[q]);
         st4(G.U0, o, hi);
         st4(G.L0, o, lo);
         st4(G.Ub, o, hi);
@@ -714,8 +676,13 @@ __global__ void k_resid(const GridDev* __restrict__ grids, const int* __restrict
     double acc[2] = {0.0, 0.0};
     for (long long q = (long long)local * blockDim.x + threadIdx.x; q < npx; q += (long long)nct * blockDim.x) {
         const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-        const double b = (double)G.b[(size_t)i * P + j];
-        const double r = b - lap_at_pair(U, L, G.wIx, G.wIy, i, j, H, W, P);
+        const size_t o = (size_t)i * P + j;
+        double b = 0.0;
+        if (j > 0) b = fma((double)G.wIx[o - 1], (double)G.gx[o - 1], b);
+        if (j < W - 1) b = fma(-(double)G.wIx[o], (double)G.gx[o], b);
+        if (i > 0) b = fma((double)G.wIy[o - P], (double)G.gy[o - P], b);
+        if (i < H - 1) b = fma(-(double)G.wIy[o], (double)G.gy[o], b);
+        const double r = resid_at_pair(U, L, G.wIx, G.wIy, G.gx, G.gy, i, j, H, W, P);
         acc[0] += r * r;
         acc[1] += b * b;
     }
@@ -763,6 +730,8 @@ cudaError_t unw_launch_row_fwd(int mode, int T, int emax, int nblk, size_t smem,
         case 0: return launch_row_fwd_t<0>(T, emax, grid, smem, s, gd, starts, n, it, cgk);
         case 1: return launch_row_fwd_t<1>(T, emax, grid, smem, s, gd, starts, n, it, cgk);
         case 2: return launch_row_fwd_t<2>(T, emax, grid, smem, s, gd, starts, n, it, cgk);
+        case 4: return launch_row_fwd_t<4>(T, emax, grid, smem, s, gd, starts, n, it, cgk);
+        case 5: return launch_row_fwd_t<5>(T, emax, grid, smem, s, gd, starts, n, it, cgk);
         default: return launch_row_fwd_t<3>(T, emax, grid, smem, s, gd, starts, n, it, cgk);
     }
 }
@@ -790,33 +759,24 @@ cudaError_t unw_launch_row_inv(int mode, int T, int emax, int nblk, size_t smem,
         case 0: return launch_row_inv_t<0>(T, emax, grid, smem, s, gd, starts, n);
         case 1: return launch_row_inv_t<1>(T, emax, grid, smem, s, gd, starts, n);
         case 2: return launch_row_inv_t<2>(T, emax, grid, smem, s, gd, starts, n);
+        case 4: return launch_row_inv_t<4>(T, emax, grid, smem, s, gd, starts, n);
         default: return launch_row_inv_t<3>(T, emax, grid, smem, s, gd, starts, n);
     }
 }
 
-template <int MODE>
-static cudaError_t launch_col_t(int T, int emax, dim3 grid, size_t smem, cudaStream_t s,
-                                const GridDev* gd, const int* st, int n) {
-#define UNW_CL(TT, EE)                                                                      \
-    if (T == TT && emax == EE) {                                                            \
-        auto kfn = k_col<TT, EE, MODE>;                                                     \
-        unw_smem_limit((const void*)kfn);                                                   \
-        kfn<<<grid, TT, smem, s>>>(gd, st, n);                                              \
-        return cudaGetLastError();                                                          \
-    }
-    UNW_CL(128, 16) UNW_CL(256, 16) UNW_CL(512, 16) UNW_CL(1024, 16) UNW_CL(1024, 32)
-#undef UNW_CL
-    return cudaErrorInvalidConfiguration;
-}
-
-cudaError_t unw_launch_col(int mode, int T, int emax, int nblk, size_t smem, cudaStream_t s,
-                           const GridDev* gd, const int* starts, int n) {
+cudaError_t unw_launch_col(int T, int nblk, size_t smem, cudaStream_t s, const GridDev* gd, const int* starts, int n) {
     if (nblk <= 0) return cudaSuccess;
-    dim3 grid(nblk);
-    switch (mode) {
-        case 0: return launch_col_t<0>(T, emax, grid, smem, s, gd, starts, n);
-        case 1: return launch_col_t<1>(T, emax, grid, smem, s, gd, starts, n);
-        default: return launch_col_t<2>(T, emax, grid, smem, s, gd, starts, n);
+    auto go = [&](auto kfn) {
+        unw_smem_limit((const void*)kfn);
+        kfn<<<nblk, T, smem, s>>>(gd, starts, n);
+        return cudaGetLastError();
+    };
+    switch (T) {
+        case 128: return go(k_col<128>);
+        case 256: return go(k_col<256>);
+        case 512: return go(k_col<512>);
+        case 1024: return go(k_col<1024>);
+        default: return cudaErrorInvalidConfiguration;
     }
 }
 

@@ -64,16 +64,15 @@ typedef struct unw_params {
                                DCT / scaling / inverse DCT of the preconditioner may run as
                                split-precision bf16 products on the tensor cores, where an
                                autotuner (timing both on the first call for a shape) finds
-                               them faster than the float32 FFT pass; unw_stats reports the
+                               them faster than the default pass; unw_stats reports the
                                choice and the float64 residual of the final system         */
 #define UNW_F_COL_TC 32     /* with UNW_F_MIXED: always the tensor-core column pass (else
                                UNW_E_UNSUPPORTED), no autotuning                             */
-#define UNW_F_COL_FFT 64    /* with UNW_F_MIXED: always the float32 FFT column pass          */
-#define UNW_F_COL_NO_TMA 128 /* power-of-two column pass at H = 2048 / 4096 with plain
-                               loads and stores, never TMA copies of the column slab (the
-                               same arithmetic and bits); by default an autotuner times both
-                               per shape on the first call and keeps the faster               */
-#define UNW_F_COL_TMA 256    /* always the TMA-staged column pass where it applies           */
+#define UNW_F_COL_FFT 64    /* with UNW_F_MIXED: always the default column pass, never the
+                               tensor cores                                                   */
+#define UNW_F_COL_NO_TMA 128 /* column pass with plain loads (the default), whatever else is set */
+#define UNW_F_COL_TMA 256    /* column pass with its tiles moved into shared memory by TMA
+                               (the same arithmetic and bits; for comparison)                 */
 #define UNW_F_MV_NO_TMA 512  /* matvec with plain loads instead of TMA-staged halo tiles (the
                                same arithmetic and bits; for comparison)                     */
 
@@ -99,10 +98,10 @@ typedef struct unw_stats {
     int32_t cg_iters[64];   /* PCG iterations of the first 64 IRLS iterations    */
     float prof_ms[16];      /* summed kernel time per family (UNW_F_PROFILE)     */
     int32_t prof_launches[16]; /* launches per family (UNW_F_PROFILE)            */
-    int32_t col_path;       /* column pass used: 0 float32 FFT, 1 tensor cores  */
-    float tune_ms[2];       /* autotuner: FFT / tensor-core column pass, ms per
+    int32_t col_path;       /* column pass used: 0 default, 1 tensor cores       */
+    float tune_ms[2];       /* autotuner: default / tensor-core column pass, ms per
                                launch (UNW_F_MIXED, 0 when not timed)          */
-    int32_t col_tma;        /* 1: the power-of-two column pass moved its slab by TMA */
+    int32_t col_tma;        /* 1: the column pass moved its tiles by TMA         */
     double resid_rel;       /* ||b - A u|| / ||b|| of the final weighted system
                                in float64 (UNW_F_MIXED; 0 otherwise): the error
                                of the result against an exact solve of the last
@@ -186,8 +185,8 @@ UNW_API int unw_apply_preconditioner(const float* r, int64_t H, int64_t W, float
 
 /* The same operator in the mixed-precision form: col_path 1 runs the column
  * DCT / scaling / inverse DCT as split-precision bf16 products on the tensor
- * cores (H <= 1024 and W a multiple of 4, else UNW_E_UNSUPPORTED), 0 the float32
- * FFT pass, -1 lets the autotuner choose.  Returns the path used (0 or 1) or a
+ * cores (H <= 1024 and W a multiple of 4, else UNW_E_UNSUPPORTED), 0 the
+ * default pass, -1 lets the autotuner choose.  Returns the path used (0 or 1) or a
  * negative error code.  It has no counterpart in the reference (which has one
  * float32 DCT path, utils_unwrap2d.py:1316-1365). */
 UNW_API int unw_apply_preconditioner_mixed(const float* r, int64_t H, int64_t W, float* z, int32_t col_path,
