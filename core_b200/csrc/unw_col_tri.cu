@@ -66,26 +66,6 @@ constexpr int TRI_HALO_A = 64, TRI_HALO_B = 32;             // halo rows of the 
 enum { TQ_RHO = 0, TQ_SEG, TQ_SEGLAST, TQ_ALL, TQ_IMG, TQ_GREEN, TQ_N };
 __host__ __device__ __forceinline__ float* tri_tab32(double* tab, int W) { return reinterpret_cast<float*>(tab + (size_t)TQ_N * W); }
 
-// Two float32 operations in one instruction (each rounded as the scalar operation).
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t.reg .b64 x, y, z, w;\n\t"
-        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("{\n\t.reg .b64 x, y, w;\n\t"
-        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "mul.rn.f32x2 w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-
 __device__ __forceinline__ uint32_t tri_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ bool tri_wait(uint64_t* bar, uint32_t parity) {

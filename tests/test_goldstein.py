@@ -94,3 +94,47 @@ def test_cuda_matches_oracle_larger_and_tensor_io():
     t = core_b200.goldstein(torch.from_numpy(z).to(dev), torch.from_numpy(c).to(dev), 32)
     assert t.is_cuda and t.dtype == torch.complex64
     np.testing.assert_array_equal(t.cpu().numpy(), out)   # deterministic
+
+
+# patch sizes and grids at which the walk changes form: every patch size, unequal sides, grids smaller
+# than a patch, one row or column, cells that end at the edge of a CTA's strip or walk, and patches that
+# are not valid; 2e-5 of the largest value as above
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,py,px,thr", [((300, 257), 4, 4, 0.5), ((130, 251), 8, 8, 0.5), ((97, 483), 16, 16, 0.5),
+                                             ((65, 225), 32, 32, 0.5), ((200, 193), 64, 64, 0.3), ((90, 300), 64, 4, 0.5),
+                                             ((70, 290), 4, 64, 0.5), ((33, 40), 32, 16, 0.5), ((129, 50), 8, 32, 0.7),
+                                             ((100, 200), 16, 64, 0.5), ((80, 99), 64, 32, 0.5), ((5, 7), 32, 32, 0.0),
+                                             ((1, 300), 16, 16, 0.02), ((300, 1), 32, 8, 0.01), ((16, 16), 16, 16, 1.0)])
+def test_cuda_matches_oracle_at_the_edges(shape, py, px, thr):
+    _gpu()
+    import core_b200
+    rng = np.random.default_rng(py * 1000 + px + shape[0])
+    z = (np.exp(1j * rng.uniform(-3, 3, shape)) * rng.uniform(0.2, 5, shape)).astype(np.complex64)
+    z[rng.random(shape) < 0.1] = np.nan
+    z[: shape[0] // 3, : shape[1] // 4] = np.nan
+    corr = rng.uniform(0, 1, shape).astype(np.float32)
+    corr[rng.random(shape) < 0.05] = np.nan
+    ref = oracle_goldstein(z, corr, py, px, thr, dtype=np.float64)
+    out = core_b200.goldstein(z, corr, py, px, threshold=thr)
+    nm = np.isnan(ref)
+    assert (np.isnan(out) == nm).all()
+    if (~nm).any():   # a single row or column has zero taper: all zeros, exactly
+        assert np.abs(out[~nm] - ref[~nm]).max() <= 2e-5 * np.abs(ref[~nm]).max()
+
+
+@pytest.mark.gpu
+def test_cuda_result_in_place_of_the_input():
+    torch = _gpu()
+    import core_b200
+    from core_b200 import _lib
+    rng = np.random.default_rng(5)
+    z = np.exp(1j * rng.uniform(-3, 3, (150, 170))).astype(np.complex64)
+    corr = rng.uniform(0, 1, z.shape).astype(np.float32)
+    ref = core_b200.goldstein(z, corr, 16)
+    dev = torch.device("cuda", 0)
+    t, c = torch.from_numpy(z).to(dev), torch.from_numpy(corr).to(dev)
+    lib = _lib.load()
+    ws = torch.empty(lib.unw_goldstein_workspace_bytes(150, 170, 16, 16), dtype=torch.uint8, device=dev)
+    _lib.check(lib.unw_goldstein_c64(t.data_ptr(), 170, c.data_ptr(), 170, 150, 170, 16, 16, 0.5, t.data_ptr(), 170,
+                                     ws.data_ptr(), ws.numel(), torch.cuda.current_stream(dev).cuda_stream))
+    np.testing.assert_array_equal(t.cpu().numpy(), ref)
