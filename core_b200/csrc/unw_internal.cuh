@@ -69,6 +69,7 @@ struct InstState {
     // post-processing (utils_unwrap2d.py:1659-1746)
     int n_nonfinite;
     int kmin, kmax;
+    int hist_base;              // cycle count of hist[0]
     int hist_ok;
     float kmed;
     float shift;

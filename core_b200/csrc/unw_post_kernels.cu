@@ -19,6 +19,17 @@ __device__ __forceinline__ bool post_ok(const InstState* st) {
     return st->n_nonfinite == 0 && st->hist_ok;
 }
 
+// Pixel kernels walk row pieces of 512 columns, a warp per piece and 32 columns per step: no
+// division per pixel, and a warp always holds adjacent pixels of one row.
+#define UNW_PIECE 512
+#define UNW_PIECES(G, local, nct)                                                                             \
+    const int np_ = ((G).W + UNW_PIECE - 1) / UNW_PIECE, lane = threadIdx.x & 31;                              \
+    for (int it_ = (local) * 8 + (int)(threadIdx.x >> 5), i = 0; it_ < (G).H * np_ && ((i = it_ / np_), true); \
+         it_ += (nct) * 8)
+#define UNW_PIECES_LOOP(G, local, nct) \
+    UNW_PIECES(G, local, nct)          \
+        for (int j0 = (it_ - i * np_) * UNW_PIECE, je_ = min(j0 + UNW_PIECE, (G).W); j0 < je_; j0 += 32)
+
 // k = round((u - phase) / 2pi) in float32, as numpy does for the reference's
 // float32 arrays (utils_unwrap2d.py:1673-1674); 2*pi rounds to 6.2831855f.
 __device__ __forceinline__ float cycles_f(float u, float ph) {
@@ -26,36 +37,63 @@ __device__ __forceinline__ float cycles_f(float u, float ph) {
 }
 
 // ---------------------------------------------------------------- stats
-// Non-finite solution count (utils_unwrap2d.py:1659-1665) and the range of the
-// cycle counts k.  An infinite input phase on a valid pixel gives k = -inf or
+// Non-finite solution count (utils_unwrap2d.py:1659-1665), range and histogram of the
+// cycle counts k in one pass.  An infinite input phase on a valid pixel gives k = -inf or
 // +inf there (u is finite by now); those are counted apart and enter the median
 // as the smallest / largest values, as they do in np.median.
+// The histogram covers |k| < hist_cap / 2 at the fixed base -hist_cap / 2 (the middle 2048 counts in
+// shared memory first); where the range does not fit that window the last CTA clears it
+// and p_hist counts again from kmin.
 __global__ void p_kstats(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
+    constexpr int SH = 2048;
     __shared__ double red[32 * 3];
-    __shared__ int smin, smax;
+    __shared__ int smin, smax, refill;
+    __shared__ int sh[SH];
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
     InstState* st = G.st;
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
-    const int W = G.W, P = G.P;
-    const long long npx = (long long)G.H * W;
+    const int P = G.P, base = -(G.hist_cap / 2);
     const float* __restrict__ U = ufinal(G, st);
-    if (threadIdx.x == 0) { smin = INT_MAX; smax = INT_MIN; }
+    if (threadIdx.x == 0) { smin = INT_MAX; smax = INT_MIN; refill = 0; }
+    for (int b = threadIdx.x; b < SH; b += blockDim.x) sh[b] = 0;
     __syncthreads();
     int kmn = INT_MAX, kmx = INT_MIN;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (long long q = (long long)local * blockDim.x + threadIdx.x; q < npx; q += (long long)nct * blockDim.x) {
-        const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-        if (!G.valid[(size_t)i * P + j]) continue;
-        const float u = U[(size_t)i * P + j];
-        if (!isfinite(u)) { acc[0] += 1.0; continue; }
-        float k = cycles_f(u, G.phase[(long long)i * G.phase_pitch + j]);
-        if (!isfinite(k)) { acc[k < 0.f ? 1 : 2] += 1.0; continue; }
-        k = fminf(fmaxf(k, -1073741824.f), 1073741824.f);
-        const int ki = (int)k;
-        kmn = min(kmn, ki);
-        kmx = max(kmx, ki);
+    UNW_PIECES_LOOP(G, local, nct) {
+        const int j = j0 + lane;
+        bool fin = false;
+        int ki = 0;
+        if (j < G.W && G.valid[(size_t)i * P + j]) {
+            const float u = U[(size_t)i * P + j];
+            if (!isfinite(u)) {
+                acc[0] += 1.0;
+            } else {
+                float k = cycles_f(u, G.phase[(long long)i * G.phase_pitch + j]);
+                if (!isfinite(k)) {
+                    acc[k < 0.f ? 1 : 2] += 1.0;
+                } else {
+                    k = fminf(fmaxf(k, -1073741824.f), 1073741824.f);
+                    ki = (int)k;
+                    kmn = min(kmn, ki);
+                    kmx = max(kmx, ki);
+                    fin = true;
+                }
+            }
+        }
+        // neighbours mostly share their count: one addition per distinct value in the warp
+        const unsigned m = __ballot_sync(0xffffffffu, fin);
+        if (fin) {
+            const int k0 = __shfl_sync(m, ki, __ffs(m) - 1);
+            const unsigned same = __all_sync(m, ki == k0) ? m : __match_any_sync(m, ki);
+            if (lane == __ffs(same) - 1) {
+                const int c = __popc(same), b = ki + SH / 2;
+                if (b >= 0 && b < SH) atomicAdd(&sh[b], c);
+                else if (ki >= base && ki - base < G.hist_cap) atomicAdd(&G.hist[ki - base], c);
+            }
+        }
+        __syncwarp();
     }
     for (int o = 16; o > 0; o >>= 1) {
         kmn = min(kmn, __shfl_down_sync(0xffffffffu, kmn, o));
@@ -63,7 +101,12 @@ __global__ void p_kstats(const GridDev* __restrict__ grids, const int* __restric
     }
     if ((threadIdx.x & 31) == 0) { atomicMin(&smin, kmn); atomicMax(&smax, kmx); }
     __syncthreads();
+    for (int b = threadIdx.x; b < SH; b += blockDim.x) {
+        const int q = b - SH / 2 - base;
+        if (sh[b] && q >= 0 && q < G.hist_cap) atomicAdd(&G.hist[q], sh[b]);
+    }
     if (threadIdx.x == 0) { atomicMin(&st->kmin, smin); atomicMax(&st->kmax, smax); }
+    __threadfence();
     if (arrive<3>(G, local, nct, acc, red)) {
         finish_sum<3>(G, nct, acc, red);
         if (threadIdx.x == 0) {
@@ -72,10 +115,15 @@ __global__ void p_kstats(const GridDev* __restrict__ grids, const int* __restric
             st->n_kpos = (int)acc[2];
             const double nfin = st->vcount - acc[1] - acc[2];
             bool ok;
+            st->hist_base = base;
             if (nfin > 0.0) {
                 const int kmin = __ldcg(&st->kmin), kmax = __ldcg(&st->kmax);
                 const long long range = (long long)kmax - (long long)kmin + 1;
                 ok = range >= 1 && range <= G.hist_cap;
+                if (kmin < base || (long long)kmax - base >= G.hist_cap) {
+                    st->hist_base = kmin;
+                    refill = ok ? 1 : 0;
+                }
             } else {
                 st->kmin = 0;  // no finite count: empty histogram
                 st->kmax = -1;
@@ -83,40 +131,30 @@ __global__ void p_kstats(const GridDev* __restrict__ grids, const int* __restric
             }
             st->hist_ok = (acc[0] == 0.0 && ok) ? 1 : 0;
         }
+        __syncthreads();
+        if (refill)
+            for (int b = threadIdx.x; b < G.hist_cap; b += blockDim.x) G.hist[b] = 0;
     }
 }
 
+// Histogram from kmin, for ranges that p_kstats's window does not hold.
 __global__ void p_hist(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
-    __shared__ int sh[2048];
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
     const InstState* st = G.st;
-    if (!post_ok(st)) return;
+    if (!post_ok(st) || st->hist_base == -(G.hist_cap / 2)) return;
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
-    const int W = G.W, P = G.P;
-    const long long npx = (long long)G.H * W;
+    const int P = G.P;
     const float* __restrict__ U = ufinal(G, st);
     const int kmin = st->kmin, range = st->kmax - st->kmin + 1;
-    if (range <= 0) return;
-    const bool small = range <= 2048;
-    if (small) {
-        for (int b = threadIdx.x; b < range; b += blockDim.x) sh[b] = 0;
-        __syncthreads();
-    }
-    for (long long q = (long long)local * blockDim.x + threadIdx.x; q < npx; q += (long long)nct * blockDim.x) {
-        const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-        if (!G.valid[(size_t)i * P + j]) continue;
+    UNW_PIECES_LOOP(G, local, nct) {
+        const int j = j0 + lane;
+        if (j >= G.W || !G.valid[(size_t)i * P + j]) continue;
         const float kf = cycles_f(U[(size_t)i * P + j], G.phase[(long long)i * G.phase_pitch + j]);
         if (!isfinite(kf)) continue;  // counted as -inf / +inf by p_kstats
         const int k = (int)kf - kmin;
-        if (k < 0 || k >= range) continue;
-        if (small) atomicAdd(&sh[k], 1); else atomicAdd(&G.hist[k], 1);
-    }
-    if (small) {
-        __syncthreads();
-        for (int b = threadIdx.x; b < range; b += blockDim.x)
-            if (sh[b]) atomicAdd(&G.hist[b], sh[b]);
+        if (k >= 0 && k < range) atomicAdd(&G.hist[k], 1);
     }
 }
 
@@ -136,13 +174,14 @@ __global__ void p_median(const GridDev* __restrict__ grids, int n) {
     const long long qlo = plo - nneg, qhi = phi - nneg;  // positions inside the histogram
     const bool need_lo = qlo >= 0 && qlo < nfin, need_hi = qhi >= 0 && qhi < nfin;
     const int range = st->kmax - st->kmin + 1;
+    const int* __restrict__ hist = G.hist + (st->kmin - st->hist_base);
     if (threadIdx.x == 0) { s_lo = -1; s_hi = -1; }
     __syncthreads();
     long long base = 0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int c0 = 0; c0 < range; c0 += blockDim.x) {
         const int b = c0 + threadIdx.x;
-        const int v = b < range ? G.hist[b] : 0;
+        const int v = b < range ? hist[b] : 0;
         int x = v;  // inclusive warp scan
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -216,6 +255,8 @@ __device__ __forceinline__ bool uf_union(int* parent, int a, int b) {
     return false;
 }
 
+// Shift and NaN restore; every valid pixel starts as a child of the first pixel of its run of
+// valid pixels within its row piece.
 __global__ void p_shift_ccinit(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
@@ -224,22 +265,32 @@ __global__ void p_shift_ccinit(const GridDev* __restrict__ grids, const int* __r
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const int W = G.W, P = G.P;
-    const long long npx = (long long)G.H * W;
     float* __restrict__ U = ufinal(G, st);
     const float sh = st->shift;
-    for (long long q = (long long)local * blockDim.x + threadIdx.x; q < npx; q += (long long)nct * blockDim.x) {
-        const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-        const size_t o = (size_t)i * P + j;
-        if (G.valid[o]) {
-            U[o] = __fsub_rn(U[o], sh);
-            G.parent[q] = (int)q;
-        } else {
-            U[o] = __int_as_float(0x7fc00000);
-            G.parent[q] = -1;
+    UNW_PIECES(G, local, nct) {
+        const int ja = (it_ - i * np_) * UNW_PIECE, je = min(ja + UNW_PIECE, W);
+        int first = i * W + ja;  // first pixel of the run that reaches this step's first column
+#pragma unroll 4
+        for (int j0 = ja; j0 < je; j0 += 32) {
+            const int j = j0 + lane;
+            const size_t o = (size_t)i * P + j;
+            const bool v = j < W && G.valid[o];
+            const unsigned m = __ballot_sync(0xffffffffu, v);
+            const int q0 = i * W + j0;
+            if (j < W) {
+                U[o] = v ? __fsub_rn(U[o], sh) : __int_as_float(0x7fc00000);
+                // lanes before this one that are not valid: the run starts after the last of them
+                const unsigned gap = ~m & ((1u << lane) - 1u);
+                G.parent[q0 + lane] = v ? (gap ? q0 + 32 - __clz(gap) : first) : -1;
+            }
+            if (m != 0xffffffffu) first = q0 + 32 - __clz(~m);
         }
     }
 }
 
+// Joins runs: across the borders of row pieces, and with the row below at the first pixel of
+// every pair of overlapping runs (further pixels of the pair would join the same two roots).
+// One join per pixel instead took most of the post-processing (4096 x 4096: 1.3 ms).
 __global__ void p_union(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
@@ -248,14 +299,21 @@ __global__ void p_union(const GridDev* __restrict__ grids, const int* __restrict
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const int H = G.H, W = G.W, P = G.P;
-    const long long npx = (long long)H * W;
     bool ok = true;
-    for (long long q = (long long)local * blockDim.x + threadIdx.x; q < npx; q += (long long)nct * blockDim.x) {
-        const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-        const size_t o = (size_t)i * P + j;
-        if (!G.valid[o]) continue;
-        if (j < W - 1 && G.valid[o + 1]) ok &= uf_union(G.parent, (int)q, (int)q + 1);
-        if (i < H - 1 && G.valid[o + P]) ok &= uf_union(G.parent, (int)q, (int)q + W);
+    UNW_PIECES(G, local, nct) {
+        const int ja = (it_ - i * np_) * UNW_PIECE, je = min(ja + UNW_PIECE, W);
+        unsigned before = 0u;  // the last column of the previous step is a valid pair
+        for (int j0 = ja; j0 < je; j0 += 32) {
+            const int j = j0 + lane;
+            const size_t o = (size_t)i * P + j;
+            const bool v = j < W && G.valid[o];
+            const bool d = v && i < H - 1 && G.valid[o + P];
+            const unsigned m = __ballot_sync(0xffffffffu, d);
+            const int q = i * W + j;
+            if (v && j == je - 1 && j < W - 1 && G.valid[o + 1]) ok &= uf_union(G.parent, q, q + 1);
+            if (d && !(((m << 1 | before) >> lane) & 1u)) ok &= uf_union(G.parent, q, q + W);
+            before = m >> 31;
+        }
     }
     if (!ok) st->hist_ok = 0;
 }
@@ -389,59 +447,57 @@ __global__ void p_accum(const GridDev* __restrict__ grids, const int* __restrict
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const int W = G.W, P = G.P;
-    const long long npx = (long long)G.H * W;
     const float* __restrict__ U = ufinal(G, st);
     const size_t cap = (size_t)G.lab_cap;
     const int nlab = st->n_labels;
     bool bad = false;
-    for (long long q0 = (long long)local * blockDim.x; q0 < npx; q0 += (long long)nct * blockDim.x) {
-        const long long q = q0 + threadIdx.x;
-        int L = 0;
-        double si = 0, ci = 0, so = 0, co = 0;
-        if (q < npx) {
-            const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-            const size_t o = (size_t)i * P + j;
-            if (G.valid[o]) {
-                L = G.lab[G.parent[q]];
-                if (L < 1 || L > nlab) { bad = true; L = 0; }
-                const float ph = G.phase[(long long)i * G.phase_pitch + j];
-                const float u = U[o];
-                si = (double)sinf(ph); ci = (double)cosf(ph);
-                so = (double)sinf(u); co = (double)cosf(u);
-            }
+    // running sums of the label that this lane is in; they go to memory when the label changes
+    int L0 = 0, cnt = 0;
+    double si = 0, ci = 0, so = 0, co = 0;
+    auto flush = [&](int L, double a, double b, double c, double d, int k) {
+        atomicAdd(&G.csum[L], a);
+        atomicAdd(&G.csum[cap + L], b);
+        atomicAdd(&G.csum[2 * cap + L], c);
+        atomicAdd(&G.csum[3 * cap + L], d);
+        atomicAdd(&G.ccount[L], k);
+    };
+    UNW_PIECES_LOOP(G, local, nct) {
+        const int j = j0 + lane;
+        const size_t o = (size_t)i * P + j;
+        if (j >= W || !G.valid[o]) continue;
+        const int q = i * W + j;
+        int L = G.lab[G.parent[q]];
+        if (L < 1 || L > nlab) { bad = true; L = 0; }
+        G.parent[q] = L;  // parent now holds the label
+        if (L == 0) continue;
+        if (L != L0) {
+            if (L0) flush(L0, si, ci, so, co, cnt);
+            L0 = L;
+            cnt = 0;
+            si = ci = so = co = 0.0;
         }
-        __syncwarp();
-        if (q < npx) {
-            const int i = (int)(q / W), j = (int)(q - (long long)i * W);
-            if (G.valid[(size_t)i * P + j]) G.parent[q] = L;  // parent now holds the label
-        }
-        const int L0 = __shfl_sync(0xffffffffu, L, 0);
-        const bool uniform = __all_sync(0xffffffffu, L == L0);
-        if (uniform) {
-            if (L0 == 0) continue;
-            int c = 1;
-            for (int o = 16; o > 0; o >>= 1) {
-                si += __shfl_down_sync(0xffffffffu, si, o);
-                ci += __shfl_down_sync(0xffffffffu, ci, o);
-                so += __shfl_down_sync(0xffffffffu, so, o);
-                co += __shfl_down_sync(0xffffffffu, co, o);
-                c += __shfl_down_sync(0xffffffffu, c, o);
-            }
-            if ((threadIdx.x & 31) == 0) {
-                atomicAdd(&G.csum[L0], si);
-                atomicAdd(&G.csum[cap + L0], ci);
-                atomicAdd(&G.csum[2 * cap + L0], so);
-                atomicAdd(&G.csum[3 * cap + L0], co);
-                atomicAdd(&G.ccount[L0], c);
-            }
-        } else if (L > 0) {
-            atomicAdd(&G.csum[L], si);
-            atomicAdd(&G.csum[cap + L], ci);
-            atomicAdd(&G.csum[2 * cap + L], so);
-            atomicAdd(&G.csum[3 * cap + L], co);
-            atomicAdd(&G.ccount[L], 1);
-        }
+        const float ph = G.phase[(long long)i * G.phase_pitch + j];
+        const float u = U[o];
+        float sn, cs;
+        sincosf(ph, &sn, &cs);
+        si += (double)sn; ci += (double)cs;
+        sincosf(u, &sn, &cs);
+        so += (double)sn; co += (double)cs;
+        cnt++;
     }
+    // the last labels of the warp: together where they are the same
+    const int Lw = __shfl_sync(0xffffffffu, L0, 0);
+    if (__all_sync(0xffffffffu, L0 == Lw)) {
+        for (int o = 16; o > 0; o >>= 1) {
+            si += __shfl_down_sync(0xffffffffu, si, o);
+            ci += __shfl_down_sync(0xffffffffu, ci, o);
+            so += __shfl_down_sync(0xffffffffu, so, o);
+            co += __shfl_down_sync(0xffffffffu, co, o);
+            cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+        }
+        if ((threadIdx.x & 31) != 0) L0 = 0;
+    }
+    if (L0) flush(L0, si, ci, so, co, cnt);
     if (bad) G.st->hist_ok = 0;
 }
 
@@ -475,11 +531,12 @@ __global__ void p_write(const GridDev* __restrict__ grids, const int* __restrict
     const int local = blockIdx.x - starts[g];
     const int nct = starts[g + 1] - starts[g];
     const int W = G.W, P = G.P;
-    const long long npx = (long long)G.H * W;
     const float* __restrict__ U = ufinal(G, st);
     const int nlab = st->n_labels;
-    for (long long q = (long long)local * blockDim.x + threadIdx.x; q < npx; q += (long long)nct * blockDim.x) {
-        const int i = (int)(q / W), j = (int)(q - (long long)i * W);
+    UNW_PIECES_LOOP(G, local, nct) {
+        const int j = j0 + lane;
+        if (j >= W) continue;
+        const int q = i * W + j;
         const size_t o = (size_t)i * P + j;
         float u = __int_as_float(0x7fc00000);
         uint16_t cc = 0;
@@ -506,6 +563,7 @@ __global__ void p_fill(const GridDev* __restrict__ grids, int n) {
     const GridDev& G = grids[g];
     const InstState* st = G.st;
     const bool failed = (G.H == 0) || st == nullptr || !post_ok(st);
+    if (!failed && G.H == G.H0 && G.W == G.W0) return;  // every pixel is inside the crop
     const long long npx = (long long)G.H0 * G.W0;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < npx; q += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(q / G.W0), j = (int)(q - (long long)i * G.W0);
