@@ -13,16 +13,6 @@ namespace {
 template <int T>
 constexpr int bl_min_blocks() { return T >= 1024 ? 1 : (1024 / T > 16 ? 16 : 1024 / T); }
 
-__device__ __forceinline__ float4 ld4v(const float* __restrict__ a, size_t o) {
-    return *reinterpret_cast<const float4*>(a + o);
-}
-__device__ __forceinline__ void st4v(float* __restrict__ a, size_t o, float4 v) {
-    *reinterpret_cast<float4*>(a + o) = v;
-}
-__device__ __forceinline__ float f4at(const float4& v, int c) {
-    return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w));
-}
-
 // x += alpha p, r -= alpha Ap at columns j..j+3 of row i (the reference's PCG
 // update, utils_unwrap2d.py:1445-1459, same operations as rowfwd_value mode 2;
 // x is the PCG correction D).
@@ -32,20 +22,20 @@ __device__ __forceinline__ float f4at(const float4& v, int c) {
 __device__ __forceinline__ float4 upd4(const GridDev& G, float* __restrict__ U, const float* __restrict__ pk,
                                        float alpha, int i, int j, int W, double (&acc)[2]) {
     const size_t o = (size_t)i * G.P + j;
-    const float4 x = ld4v(U, o), p = ld4v(pk, o), r = ld4v(G.r, o), ap = ld4v(G.Ap, o);
+    const float4 x = ld4f(U, o), p = ld4f(pk, o), r = ld4f(G.r, o), ap = ld4f(G.Ap, o);
     float4 xn, rn;
     xn.x = fmaf(alpha, p.x, x.x); xn.y = fmaf(alpha, p.y, x.y);
     xn.z = fmaf(alpha, p.z, x.z); xn.w = fmaf(alpha, p.w, x.w);
     rn.x = fmaf(-alpha, ap.x, r.x); rn.y = fmaf(-alpha, ap.y, r.y);
     rn.z = fmaf(-alpha, ap.z, r.z); rn.w = fmaf(-alpha, ap.w, r.w);
-    st4v(U, o, xn);
-    st4v(G.r, o, rn);
+    st4f(U, o, xn);
+    st4f(G.r, o, rn);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         if (j + c < W) {
-            const float v = f4at(rn, c);
+            const float v = f4get(rn, c);
             acc[0] += (double)v * (double)v;
-            acc[1] += isfinite(f4at(xn, c)) ? 0.0 : 1.0;
+            acc[1] += isfinite(f4get(xn, c)) ? 0.0 : 1.0;
         }
     }
     return rn;
@@ -83,13 +73,16 @@ __global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL::T, MODE>())) k_rowf
         const int i0 = 2 * pair, i1 = i0 + 1;
         const bool has1 = i1 < H;
         __syncthreads();  // previous row pair's reads of sm are done
-        if (MODE == 2) {
+        if (MODE == 1 || MODE == 2) {
             for (int j = 4 * t; j < W; j += 4 * T) {
-                const float4 a = upd4(G, U, pk, alpha, i0, j, W, acc);
-                const float4 b = has1 ? upd4(G, U, pk, alpha, i1, j, W, acc) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 a = MODE == 1 ? rowf_start4(G, U, Lo, i0, j, acc) : upd4(G, U, pk, alpha, i0, j, W, acc);
+                const float4 b = !has1 ? z
+                                 : MODE == 1 ? rowf_start4(G, U, Lo, i1, j, acc)
+                                             : upd4(G, U, pk, alpha, i1, j, W, acc);
 #pragma unroll
                 for (int c = 0; c < 4; c++)
-                    if (j + c < W) sm[BL::pos(mk_perm(j + c, W))] = make_float2(f4at(a, c), f4at(b, c));
+                    if (j + c < W) sm[BL::pos(mk_perm(j + c, W))] = make_float2(f4get(a, c), f4get(b, c));
             }
         } else {
             for (int j = t; j < W; j += T) {
@@ -166,13 +159,13 @@ __global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const
                     zb[c] = -v.y;
                 }
                 const size_t oa = (size_t)i0 * P + j;
-                const float4 pa = ld4v(G.p0, oa);
-                st4v(G.p0, oa, make_float4(fadd(fmul(pa.x, beta), za[0]), fadd(fmul(pa.y, beta), za[1]),
+                const float4 pa = ld4f(G.p0, oa);
+                st4f(G.p0, oa, make_float4(fadd(fmul(pa.x, beta), za[0]), fadd(fmul(pa.y, beta), za[1]),
                                            fadd(fmul(pa.z, beta), za[2]), fadd(fmul(pa.w, beta), za[3])));
                 if (has1) {
                     const size_t ob = oa + P;
-                    const float4 pb = ld4v(G.p0, ob);
-                    st4v(G.p0, ob, make_float4(fadd(fmul(pb.x, beta), zb[0]), fadd(fmul(pb.y, beta), zb[1]),
+                    const float4 pb = ld4f(G.p0, ob);
+                    st4f(G.p0, ob, make_float4(fadd(fmul(pb.x, beta), zb[0]), fadd(fmul(pb.y, beta), zb[1]),
                                                fadd(fmul(pb.z, beta), zb[2]), fadd(fmul(pb.w, beta), zb[3])));
                 }
             }

@@ -21,16 +21,6 @@ constexpr int min_blocks() { return T >= 1024 ? 1 : (1024 / T > 16 ? 16 : 1024 /
 
 __device__ __forceinline__ int mk_pos(int n, int N) { return (n & 1) ? N - 1 - (n >> 1) : (n >> 1); }
 
-__device__ __forceinline__ float4 ld4f(const float* __restrict__ a, size_t o) {
-    return *reinterpret_cast<const float4*>(a + o);
-}
-__device__ __forceinline__ void st4f(float* __restrict__ a, size_t o, float4 v) {
-    *reinterpret_cast<float4*>(a + o) = v;
-}
-__device__ __forceinline__ float f4get(const float4& v, int c) {
-    return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w));
-}
-
 // Four consecutive source values of row i (columns j..j+3) of the row-forward pass.
 template <int MODE>
 __device__ __forceinline__ float4 rowf_vals4(const GridDev& G, float* __restrict__ U, const float* __restrict__ Lo,
@@ -52,44 +42,7 @@ __device__ __forceinline__ float4 rowf_vals4(const GridDev& G, float* __restrict
     } else if (MODE == 3) {
         return ld4f(G.r, o);
     } else if (MODE == 1) {
-        // r = b - A x0 at columns j..j+3 in divergence form (resid_at_pair)
-        const int H = G.H, W = G.W, P = G.P;
-        const float4 x4 = ld4f(U, o), l4 = ld4f(Lo, o), wx4 = ld4f(G.wIx, o), wy4 = ld4f(G.wIy, o);
-        const float4 gx4 = ld4f(G.gx, o), gy4 = ld4f(G.gy, o);
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 xu4 = i > 0 ? ld4f(U, o - P) : z4, lu4 = i > 0 ? ld4f(Lo, o - P) : z4;
-        const float4 wyu4 = i > 0 ? ld4f(G.wIy, o - P) : z4, gyu4 = i > 0 ? ld4f(G.gy, o - P) : z4;
-        const float4 xd4 = i < H - 1 ? ld4f(U, o + P) : z4, ld4 = i < H - 1 ? ld4f(Lo, o + P) : z4;
-        const float xl = j > 0 ? U[o - 1] : 0.f, ll = j > 0 ? Lo[o - 1] : 0.f;
-        const float wxl = j > 0 ? G.wIx[o - 1] : 0.f, gxl = j > 0 ? G.gx[o - 1] : 0.f;
-        const float xr = j + 4 < W ? U[o + 4] : 0.f, lr = j + 4 < W ? Lo[o + 4] : 0.f;
-        const double xs[6] = {pair_val(xl, ll), pair_val(x4.x, l4.x), pair_val(x4.y, l4.y), pair_val(x4.z, l4.z),
-                              pair_val(x4.w, l4.w), pair_val(xr, lr)};
-        const float wxs[5] = {wxl, wx4.x, wx4.y, wx4.z, wx4.w};
-        const float gxs[5] = {gxl, gx4.x, gx4.y, gx4.z, gx4.w};
-        float out[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int jj = j + q;
-            const double xc = xs[q + 1];
-            double r = 0.0;
-            if (jj > 0) r = fma((double)wxs[q], (double)gxs[q] - (xc - xs[q]), r);
-            if (jj < W - 1) r = fma(-(double)wxs[q + 1], (double)gxs[q + 1] - (xs[q + 2] - xc), r);
-            if (i > 0)
-                r = fma((double)f4get(wyu4, q),
-                        (double)f4get(gyu4, q) - (xc - pair_val(f4get(xu4, q), f4get(lu4, q))), r);
-            if (i < H - 1)
-                r = fma(-(double)f4get(wy4, q),
-                        (double)f4get(gy4, q) - (pair_val(f4get(xd4, q), f4get(ld4, q)) - xc), r);
-            const float val = (float)r;
-            out[q] = val;
-            acc[0] += isfinite(val) ? 0.0 : 1.0;
-            acc[1] += (double)val * (double)val;
-        }
-        const float4 r4 = make_float4(out[0], out[1], out[2], out[3]);
-        st4f(G.r, o, r4);
-        st4f(G.D, o, z4);
-        return r4;
+        return rowf_start4(G, U, Lo, i, j, acc);
     } else {
         float4 v;
         v.x = rowfwd_value<MODE>(G, U, Lo, pk, alpha, i, j, acc);
