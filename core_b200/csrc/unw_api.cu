@@ -693,7 +693,9 @@ int prepare(Solver& S, const std::vector<int>& idx, const unw_grid* grids, const
         GridDev& G = S.hg[g];
         if (G.H == 0) continue;
         CK(unw_launch_tables(G.prow.fft, G.prow, const_cast<float*>(G.sW), G.W, s));
-        if (G.prow.blue) CK(unw_launch_hspec(pick_threads(prow[g].n, prow[g].cap), prow[g].emax, G.prow, s));
+        if (G.prow.blue)
+            CK(unw_launch_hspec(pick_threads(prow[g].n, prow[g].cap), prow[g].emax, G.prow,
+                                S.sh.row_bl % 3 ? 0 : S.sh.row_bl / 3, s));
         CK(unw_tri_tables(const_cast<double*>(G.tri), G.H, G.W, s));
         // column eigenvalue parts of the tensor-core pass (no transform tables: empty plan)
         if (tc_h > 0) CK(unw_launch_tables(FftPlanDev{}, DctPlanDev{}, const_cast<float*>(G.sH), G.H, s));

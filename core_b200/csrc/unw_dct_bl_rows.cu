@@ -10,8 +10,13 @@
 
 namespace {
 
-template <int T>
-constexpr int bl_min_blocks() { return T >= 1024 ? 1 : (1024 / T > 16 ? 16 : 1024 / T); }
+// resident CTAs to compile for: 768 threads per SM (80 registers) where the transforms keep their ends in
+// registers, else 1024
+template <class BL>
+constexpr int bl_min_blocks() {
+    constexpr int n = (BL::FUSED ? 768 : 1024) / BL::T;
+    return n < 1 ? 1 : (n > 16 ? 16 : n);
+}
 
 // x += alpha p, r -= alpha Ap at columns j..j+3 of row i (the reference's PCG
 // update, utils_unwrap2d.py:1445-1459, same operations as rowfwd_value mode 2;
@@ -41,15 +46,15 @@ __device__ __forceinline__ float4 upd4(const GridDev& G, float* __restrict__ U, 
     return rn;
 }
 
-// the PCG-start pass (mode 1, once per IRLS iteration) takes half the resident CTAs for
-// the registers of the iterate pair's stencil
-template <int T, int MODE>
+// the PCG-start pass (mode 1, once per IRLS iteration) is compiled for 512 threads per SM: the iterate
+// pair's stencil takes up to 128 registers
+template <class BL, int MODE>
 constexpr int bl_rowf_blocks() {
-    return MODE == 1 ? (bl_min_blocks<T>() / 2 > 0 ? bl_min_blocks<T>() / 2 : 1) : bl_min_blocks<T>();
+    return MODE == 1 ? (BL::T > 512 ? 1 : 512 / BL::T > 8 ? 8 : 512 / BL::T) : bl_min_blocks<BL>();
 }
 
 template <class BL, int MODE>
-__global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL::T, MODE>())) k_rowf_bl(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL, MODE>())) k_rowf_bl(const GridDev* __restrict__ grids,
                                                                            const int* __restrict__ starts, int n,
                                                                            int it, int cgk) {
     constexpr int T = BL::T;
@@ -68,7 +73,10 @@ __global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL::T, MODE>())) k_rowf
     const float* pk = (MODE == 2) ? G.p0 : nullptr;
     const float alpha = (MODE == 2) ? st->alpha : 0.f;
     const float2* __restrict__ dw = G.prow.dctw;
+    const float2* __restrict__ ch = G.prow.chirp;
     double acc[2] = {0.0, 0.0};
+    // sequence position m of a row pair's values, with the input chirp
+    auto put = [&](int m, float a, float b) { sm[BL::pos(m)] = cmul(make_float2(a, b), cconj(__ldg(&ch[m]))); };
     for (int pair = local; pair < (H + 1) / 2; pair += nct) {
         const int i0 = 2 * pair, i1 = i0 + 1;
         const bool has1 = i1 < H;
@@ -82,13 +90,13 @@ __global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL::T, MODE>())) k_rowf
                                              : upd4(G, U, pk, alpha, i1, j, W, acc);
 #pragma unroll
                 for (int c = 0; c < 4; c++)
-                    if (j + c < W) sm[BL::pos(mk_perm(j + c, W))] = make_float2(f4get(a, c), f4get(b, c));
+                    if (j + c < W) put(mk_perm(j + c, W), f4get(a, c), f4get(b, c));
             }
         } else {
             for (int j = t; j < W; j += T) {
                 const float a = rowfwd_value<MODE>(G, U, Lo, pk, alpha, i0, j, acc);
                 const float b = has1 ? rowfwd_value<MODE>(G, U, Lo, pk, alpha, i1, j, acc) : 0.f;
-                sm[BL::pos(mk_perm(j, W))] = make_float2(a, b);
+                put(mk_perm(j, W), a, b);
             }
         }
         __syncthreads();
@@ -114,7 +122,7 @@ __global__ void __launch_bounds__(BL::T, (bl_rowf_blocks<BL::T, MODE>())) k_rowf
 }
 
 template <class BL, int MODE>
-__global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(BL::T, bl_min_blocks<BL>()) k_rowi_bl(const GridDev* __restrict__ grids,
                                                                            const int* __restrict__ starts, int n) {
     constexpr int T = BL::T;
     extern __shared__ float2 sm[];
@@ -128,6 +136,7 @@ __global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const
     const int H = G.H, W = G.W, P = G.P;
     const int t = threadIdx.x;
     const float2* __restrict__ dw = G.prow.dctw;
+    const float2* __restrict__ ch = G.prow.chirp;
     const float beta = MODE == 2 ? st->beta : 0.f;
     double acc[2] = {0.0, 0.0};
     for (int pair = local; pair < (H + 1) / 2; pair += nct) {
@@ -136,7 +145,7 @@ __global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const
         const float* __restrict__ Ta = G.Tz + (size_t)i0 * P;
         const float* __restrict__ Tb = G.Tz + (size_t)i1 * P;
         __syncthreads();  // previous row pair's reads of sm are done
-        // DCT-III pre-twiddle: V'_k = conj(w_k) (Y_k - i Y_{W-k}), Y_W = 0; store conj(C')
+        // DCT-III pre-twiddle: V'_k = conj(w_k) (Y_k - i Y_{W-k}), Y_W = 0; store conj(C') with the chirp
         for (int k = t; k < W; k += T) {
             const float ya = Ta[k], yb = has1 ? Tb[k] : 0.f;
             const float yam = k ? Ta[W - k] : 0.f;
@@ -144,7 +153,7 @@ __global__ void __launch_bounds__(BL::T, bl_min_blocks<BL::T>()) k_rowi_bl(const
             const float2 wc = cconj(__ldg(&dw[k]));
             const float2 Pa = cmul(wc, make_float2(ya, -yam));
             const float2 Pb = cmul(wc, make_float2(yb, -ybm));
-            sm[BL::pos(k)] = cconj(make_float2(Pa.x - Pb.y, Pa.y + Pb.x));
+            sm[BL::pos(k)] = cconj(cmul(make_float2(Pa.x - Pb.y, Pa.y + Pb.x), __ldg(&ch[k])));
         }
         __syncthreads();
         BL::dft(sm, t, W, G.prow);

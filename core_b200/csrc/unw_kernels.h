@@ -61,7 +61,7 @@ int unw_set_error(int code, const char* msg);
 // solver kernels
 cudaError_t unw_launch_tables(const FftPlanDev& f, const DctPlanDev& d, float* sv, int Ncos,
                               cudaStream_t s);
-cudaError_t unw_launch_hspec(int T, int emax, const DctPlanDev& d, cudaStream_t s);
+cudaError_t unw_launch_hspec(int T, int emax, const DctPlanDev& d, int m3, cudaStream_t s);
 cudaError_t unw_launch_row_fwd(int mode, int T, int emax, int nblk, size_t smem, cudaStream_t s,
                                const GridDev* gd, const int* starts, int n, int it, int cgk);
 cudaError_t unw_launch_row_inv(int mode, int T, int emax, int nblk, size_t smem, cudaStream_t s,

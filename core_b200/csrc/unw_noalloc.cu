@@ -210,9 +210,9 @@ extern "C" int unw_apply_preconditioner_noalloc(const float* r, int64_t H, int64
     if ((e = unw_launch_tables(G.prow.fft, G.prow, const_cast<float*>(G.sW), G.W, s)) != cudaSuccess ||
         (e = unw_launch_tables(G.pcol.fft, G.pcol, const_cast<float*>(G.sH), G.H, s)) != cudaSuccess)
         return unw_set_error(UNW_E_CUDA, cudaGetErrorString(e));
-    if (G.prow.blue && (e = unw_launch_hspec(pick_threads(pr.n, pr.cap), 16, G.prow, s)) != cudaSuccess)
+    if (G.prow.blue && (e = unw_launch_hspec(pick_threads(pr.n, pr.cap), 16, G.prow, 0, s)) != cudaSuccess)
         return unw_set_error(UNW_E_CUDA, cudaGetErrorString(e));
-    if (G.pcol.blue && (e = unw_launch_hspec(pick_threads(pc.n, pc.cap), 16, G.pcol, s)) != cudaSuccess)
+    if (G.pcol.blue && (e = unw_launch_hspec(pick_threads(pc.n, pc.cap), 16, G.pcol, 0, s)) != cudaSuccess)
         return unw_set_error(UNW_E_CUDA, cudaGetErrorString(e));
     const size_t row_smem = (size_t)pr.n * sizeof(float2), col_smem = (size_t)nseq * pc.n * sizeof(float2);
     e = row_p2 ? unw_launch_rowf_p2(row_p2, 3, n_row, s, dG, dS + 2 * KS_ROWPAIR, 1, 0, 0)

@@ -123,20 +123,21 @@ __device__ __forceinline__ void smem_fft_rec(float2* sm, int t, const float2* tw
     }
 }
 
-template <int N, int P, int NS, bool IN_REG, bool OUT_REG>
+template <int N, int P, int NS, bool IN_REG, bool OUT_REG, int TS>
 __device__ __forceinline__ void io_fft_rec(float2 (&v)[16], float2* sm, int t, const float2* tw) {
     if constexpr (P < RegFft<N>::NPASS) {
         constexpr int R = (P < RegFft<N>::NP16) ? 16 : (1 << RegFft<N>::REM);
-        reg_pass<N, R, NS, IN_REG && P == 0, OUT_REG && P == RegFft<N>::NPASS - 1>(v, sm, t, tw);
-        io_fft_rec<N, P + 1, NS * R, IN_REG, OUT_REG>(v, sm, t, tw);
+        reg_pass<N, R, NS, IN_REG && P == 0, OUT_REG && P == RegFft<N>::NPASS - 1, TS>(v, sm, t, tw);
+        io_fft_rec<N, P + 1, NS * R, IN_REG, OUT_REG, TS>(v, sm, t, tw);
     }
 }
 
 // Forward FFT with the input in registers (stride-T layout) or in shared memory
 // (natural order), and the output likewise; the other side goes through `sm`.
-template <int N, bool IN_REG, bool OUT_REG>
+// TS > 1: `tw` is the table of a TS times longer transform.
+template <int N, bool IN_REG, bool OUT_REG, int TS = 1>
 __device__ __forceinline__ void io_fft(float2 (&v)[16], float2* sm, int t, const float2* tw) {
-    io_fft_rec<N, 0, 1, IN_REG, OUT_REG>(v, sm, t, tw);
+    io_fft_rec<N, 0, 1, IN_REG, OUT_REG, TS>(v, sm, t, tw);
 }
 
 // Forward FFT of the sequence held in shared memory (natural order, padded

@@ -50,9 +50,10 @@ __global__ void k_tables(FftPlanDev f, DctPlanDev d, float* sv, int Ncos) {
     }
 }
 
-// Bluestein filter spectrum hspec = FFT_M(h) / M, h_j = chirp_|j| for |j| < N.
+// Bluestein filter spectrum hspec = FFT_M(h) / M, h_j = chirp_|j| for |j| < N; in natural order, or
+// with m3 = M / 3 > 0 as [s][k], entry 3 k + s (the order of blue_fft3).
 template <int T, int EMAX>
-__global__ void __launch_bounds__(T) k_hspec(DctPlanDev d) {
+__global__ void __launch_bounds__(T) k_hspec(DctPlanDev d, int m3) {
     extern __shared__ float2 sm[];
     const int M = d.fft.n, N = d.N;
     for (int m = threadIdx.x; m < M; m += T) {
@@ -65,7 +66,10 @@ __global__ void __launch_bounds__(T) k_hspec(DctPlanDev d) {
     fft_smem<T, EMAX>(sm, 1, M, d.fft);
     float2* hs = const_cast<float2*>(d.hspec);
     const float inv = 1.0f / (float)M;
-    for (int m = threadIdx.x; m < M; m += T) hs[m] = make_float2(sm[m].x * inv, sm[m].y * inv);
+    for (int m = threadIdx.x; m < M; m += T) {
+        const int e = m3 ? 3 * (m % m3) + m / m3 : m;
+        hs[m] = make_float2(sm[e].x * inv, sm[e].y * inv);
+    }
 }
 
 // ============================================================ state / setup
@@ -796,13 +800,13 @@ cudaError_t unw_launch_tables(const FftPlanDev& f, const DctPlanDev& d, float* s
     return cudaGetLastError();
 }
 
-cudaError_t unw_launch_hspec(int T, int emax, const DctPlanDev& d, cudaStream_t s) {
+cudaError_t unw_launch_hspec(int T, int emax, const DctPlanDev& d, int m3, cudaStream_t s) {
     const size_t smem = (size_t)d.fft.n * sizeof(float2);
 #define UNW_HS(TT, EE)                                                                      \
     if (T == TT && emax == EE) {                                                            \
         auto kfn = k_hspec<TT, EE>;                                                         \
         unw_smem_limit((const void*)kfn);                                                   \
-        kfn<<<1, TT, smem, s>>>(d);                                                         \
+        kfn<<<1, TT, smem, s>>>(d, m3);                                                     \
         return cudaGetLastError();                                                          \
     }
     UNW_HS(128, 16) UNW_HS(256, 16) UNW_HS(512, 16) UNW_HS(1024, 16) UNW_HS(1024, 32)
