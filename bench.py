@@ -343,9 +343,9 @@ def run_b200(args):
              "col_path": int(st_mixed.col_path), "resid_rel": float(f"{st_mixed.resid_rel:.3g}"),
              "ratio_mixed_over_plain": round(t_dev / args.steps / t_mixed, 4),
              "plain_no_graph": {"value": round(npx / 1e6 / t_nograph, 3), "ms_per_step": round(t_nograph * 1e3, 3)},
-             "note": (f"H = {H} > 1024: the mixed form keeps the float32 FFT column pass (the tensor-core "
+             "note": (f"H = {H} > 1024: the mixed form keeps the default column pass (the tensor-core "
                       "pass covers grids of at most 1024 rows); see mixed_1024 for where it applies")
-             if H > 1024 else "H <= 1024: the autotuner chose col_path (0 FFT, 1 tensor cores)"}
+             if H > 1024 else "H <= 1024: the autotuner chose col_path (0 default, 1 tensor cores)"}
 
     # ---- per-kernel CUDA-event times (UNW_F_PROFILE brackets every launch with an event
     # pair on the solve stream; the events add about 10 us per launch, so this timed pass
@@ -432,19 +432,6 @@ def run_b200(args):
                 "timing": f"per-launch CUDA events on the solve stream over a separate timed pass of "
                           f"{prof_steps} step(s) ({t_prof * 1e3:.1f} ms/step with the events)"}
 
-    # column pass: bound by instruction issue, not memory -> also its issue-rate roofline
-    # (warp instructions per launch from the ncu capture in profiles/, peak = 4 issue slots
-    # per SM per cycle at the sampled SM clock)
-    if os.path.exists(tf):
-        inst = json.load(open(tf)).get("inst", {}).get("col")
-        if inst and fam["col"][1]:
-            col_s = fam["col"][0] / 1e3 / fam["col"][1]
-            sm_mhz = (clk or {}).get("sm_mhz") or 1965.0
-            peak_i = 148 * 4 * sm_mhz * 1e6 / 1e9
-            roofline["col_issue"] = {"bound": "issue", "kernel": "col", "unit": "Ginst/s (warp)",
-                                     "inst_per_launch": inst, "achieved": round(inst / col_s / 1e9, 1),
-                                     "peak": round(peak_i, 1), "frac": round(inst / col_s / 1e9 / peak_i, 4)}
-
     # ---- the 64-grid uneven stack (the other workload of the headline metric), sharded by grid
     stack = None
     if not args.no_stack_line:
@@ -475,7 +462,7 @@ def run_b200(args):
                            "ratio_mixed_over_plain": round(m_val / s_val, 4),
                            "tensor_core_grids": int(sum(m_paths)),
                            "note": "every stack grid has more than 1024 rows, so the mixed form keeps the "
-                                   "float32 FFT column pass (the tensor-core pass covers H <= 1024)"},
+                                   "default column pass (the tensor-core pass covers H <= 1024)"},
                  "kernels": {"note": "per-launch CUDA-event times of one separately profiled batched solve of "
                                      "this rank's grids (launch groups one after another; the timed steps run "
                                      "them concurrently)", **s_prof},

@@ -79,11 +79,11 @@ COL_PASSES = ("auto", "tc", "fft")
 def precision_flags(precision="plain", col_pass="auto"):
     """UNW_F_* bits of the precision keywords.
 
-    precision='plain'  float32 FFT DCTs throughout (the reference's arithmetic);
+    precision='plain'  the default passes: float32 row transforms, tridiagonal column solves;
     precision='mixed'  for grids of at most 1024 rows the column DCT / scaling /
                        inverse DCT of the preconditioner may run as split-precision
                        bf16 products on the tensor cores: col_pass='auto' lets the
-                       autotuner time both on the first call for a shape, 'tc' / 'fft'
+                       autotuner time both on the first call for a shape, 'tc' / 'fft' (the default pass)
                        force one; the stats report the path and the float64 residual of
                        the final weighted system.
     """
@@ -224,7 +224,7 @@ def irls_unwrap_2d(phase, weight=None, device='auto', max_iter=50, tol=1e-3,
       check_every   IRLS iterations enqueued between device->host convergence reads
       fixed_iters   run exactly max_iter x cg_max_iter iterations (tol / cg_tol stop
                     tests off, numerical breaks kept): identical work for timing
-      precision     'plain' (float32 FFT DCTs) or 'mixed' (tensor-core column pass for
+      precision     'plain' (the default passes) or 'mixed' (tensor-core column pass for
                     grids of <= 1024 rows where the autotuner finds it faster)
       col_pass      with precision='mixed': 'auto', or force 'tc' / 'fft'
     """
