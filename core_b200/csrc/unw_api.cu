@@ -242,8 +242,9 @@ struct Shape {
     int mv_tma = 0;               // matvec on TMA-staged halo tiles
 };
 
-int elem_ctas(long long npx) {
-    long long c = (npx + 2047) / 2048;
+// CTAs of the elementwise kernels: a row piece per warp (eight warps) up to the cap
+int elem_ctas(long long H, long long W) {
+    const long long c = (H * ((W + UNW_ELEM_PIECE - 1) / UNW_ELEM_PIECE) + 7) / 8;
     return (int)std::max<long long>(1, std::min<long long>(c, ELEM_MAX_CTAS));
 }
 
@@ -327,7 +328,7 @@ int kind_ctas(const GridDev& G, int kind) {
         case KS_COL: return G.col_ctas;
         case KS_STEN: return std::min(G.sten_tiles_x * ((G.H + 8 * G.sten_rows - 1) / (8 * G.sten_rows)), CTAS_HEAD);
         case KS_MATVEC: return std::min(G.sten_tiles_x * ((G.H + 15) / 16), CTAS_MATVEC);
-        case KS_ELEM: return elem_ctas(npx);
+        case KS_ELEM: return elem_ctas(G.H, G.W);
         case KS_ONE: return 1;
         default: return (int)((npx + 4095) / 4096);  // post tiles
     }

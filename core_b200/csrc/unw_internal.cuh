@@ -149,6 +149,9 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 
+// columns of a row that a warp of the elementwise kernels takes at a time
+#define UNW_ELEM_PIECE 256
+
 // Two float32 operations in one instruction (each rounded as the scalar operation).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 d;

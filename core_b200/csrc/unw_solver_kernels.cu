@@ -93,6 +93,18 @@ __global__ void k_state_init(const GridDev* __restrict__ grids, int n, UnwScalar
     *grids[g].counter = 0u;
 }
 
+// Walk of the elementwise kernels (KS_ELEM): a warp takes row pieces of UNW_ELEM_PIECE columns, a lane V
+// adjacent columns per step; P is a multiple of 4, so a group of four starting below W stays in the row.
+// Rows dealt to whole CTAs left most threads of a narrow grid idle and a small grid's CTAs with a
+// dozen rows one after another: 200 x 180, us per launch, then / now: k_mean 10.0 / 5.7, k_rel 12.6 / 7.2; at
+// 1024 x 1024 7.2 / 7.5 and 9.7 / 12.0; bound there and above by the bytes.
+#define UNW_PIECES_LOOP(G, local, nct, V)                                                                       \
+    for (int np_ = ((G).W + UNW_ELEM_PIECE - 1) / UNW_ELEM_PIECE, q_ = (local) * 8 + (int)(threadIdx.x >> 5), i = 0; \
+         q_ < (G).H * np_ && ((i = q_ / np_), true); q_ += (nct) * 8)                                           \
+        for (int j0_ = (q_ - i * np_) * UNW_ELEM_PIECE, je_ = min(j0_ + UNW_ELEM_PIECE, (G).W),                 \
+                 j = j0_ + (V) * (int)(threadIdx.x & 31);                                                       \
+             j < je_; j += 32 * (V))
+
 // NaN fill, weight clipping, wrapped gradients and edge weights
 // (utils_unwrap2d.py:1228-1241, :1254-1262, :1267-1275).  KS_ELEM shape.
 //
@@ -125,8 +137,7 @@ __global__ void k_setup(const GridDev* __restrict__ grids, const int* __restrict
     const int nct = starts[g + 1] - starts[g];
     const int H = G.H, W = G.W, P = G.P;
     double acc[1] = {0.0};
-    for (int i = local; i < H; i += nct)
-    for (int j = threadIdx.x; j < W; j += blockDim.x) {
+    UNW_PIECES_LOOP(G, local, nct, 1) {
         float ph, w, phr, wr, phd, wd;
         bool v, vr, vd;
         px_in(G, i, j, ph, w, v);
@@ -540,11 +551,6 @@ __global__ void __launch_bounds__(256, 4) k_head(const GridDev* __restrict__ gri
 }
 
 // ============================================================ elementwise kernels (KS_ELEM)
-// A CTA takes whole rows (grid-stride over rows), threads take float4 column
-// groups; P is a multiple of 4, so a group starting below W stays in the row.
-#define UNW_ROWS_LOOP(G, local, nct)                          \
-    for (int i = (local); i < (G).H; i += (nct))              \
-        for (int j = 4 * threadIdx.x; j < (G).W; j += 4 * blockDim.x)
 
 // sum over all pixels of u * valid (utils_unwrap2d.py:1539-1541), u = U + L in float64
 __global__ void k_mean(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n, int it) {
@@ -558,7 +564,7 @@ __global__ void k_mean(const GridDev* __restrict__ grids, const int* __restrict_
     const float* __restrict__ uc = (it & 1) ? G.U1 : G.U0;
     const float* __restrict__ lc = (it & 1) ? G.L1 : G.L0;
     double acc[1] = {0.0};
-    UNW_ROWS_LOOP(G, local, nct) {
+    UNW_PIECES_LOOP(G, local, nct, 4) {
         const size_t o = (size_t)i * G.P + j;
         const F4 u = ld4(uc, o), l = ld4(lc, o);
         const uchar4 v = *reinterpret_cast<const uchar4*>(G.valid + o);
@@ -583,7 +589,7 @@ __global__ void k_init_recentre(const GridDev* __restrict__ grids, const int* __
     const int nct = starts[g + 1] - starts[g];
     const double m = st->vcount > 0 ? st->mean : 0.0;
     const bool refined = !(st->status & 1);  // L0 is written unless the initial solution was non-finite
-    UNW_ROWS_LOOP(G, local, nct) {
+    UNW_PIECES_LOOP(G, local, nct, 4) {
         const size_t o = (size_t)i * G.P + j;
         const F4 u = ld4(G.U0, o);
         F4 l{}, hi, lo;
@@ -607,7 +613,7 @@ __global__ void k_copy_best(const GridDev* __restrict__ grids, const int* __rest
     const int nct = starts[g + 1] - starts[g];
     const float* __restrict__ un = (it & 1) ? G.U0 : G.U1;
     const float* __restrict__ ln = (it & 1) ? G.L0 : G.L1;
-    UNW_ROWS_LOOP(G, local, nct) {
+    UNW_PIECES_LOOP(G, local, nct, 4) {
         const size_t o = (size_t)i * G.P + j;
         st4(G.Ub, o, ld4(un, o));
         st4(G.Lb, o, ld4(ln, o));
@@ -630,7 +636,7 @@ __global__ void k_rel(const GridDev* __restrict__ grids, const int* __restrict__
     float* __restrict__ un = (it & 1) ? G.U0 : G.U1;
     float* __restrict__ ln = (it & 1) ? G.L0 : G.L1;
     double acc[3] = {0.0, 0.0, 0.0};
-    UNW_ROWS_LOOP(G, local, nct) {
+    UNW_PIECES_LOOP(G, local, nct, 4) {
         const size_t o = (size_t)i * G.P + j;
         const F4 uh = ld4(un, o), ul = ld4(ln, o), dd = ld4(G.D, o), vh = ld4(up, o), vl = ld4(lp, o);
         F4 nh, nl;
