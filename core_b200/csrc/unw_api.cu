@@ -499,7 +499,8 @@ std::array<int, 4> group_key(int H, int W, int flags) {
     else if (bl_len(W)) { k[0] = 2; k[1] = bl_len(W); }
     else { const HostPlan hp = make_plan(W); k[0] = 0; k[1] = pick_threads(hp.n, hp.cap) * 64 + hp.emax; }
     k[2] = unw_tri_rows(H, W);
-    if (flags & UNW_F_MIXED) k[3] = H;  // the tensor-core column pass needs one H per launch
+    // the tensor-core column pass needs one H per launch
+    if ((flags & UNW_F_MIXED) && H <= UNW_TC_MAX_H) k[3] = H;
     return k;
 }
 
