@@ -141,6 +141,8 @@ __device__ __noinline__ float gs_pow(float2 F, float alpha) {
     return powf(fmaxf(sqrtf(F.x * F.x + F.y * F.y), 1e-10f), alpha);
 }
 
+__device__ __noinline__ float2 gs_third(float2 s) { return make_float2(s.x / 3.f, s.y / 3.f); }
+
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // PX threads per patch.  Patches of at most 32 columns lie inside a warp.
@@ -305,20 +307,23 @@ __global__ void __launch_bounds__(256, (GsShape<PY, PX>::CTAS)) k_gs_walk(GsArgs
         // normalisation and NaN restore (:308-320)
         if (pi >= i0 && slot > 0 && c < SX && x < a.nx) {
             const int n = own + cover[buf][slot - 1];
-            // s / n by the reciprocal and one correction (correctly rounded: n is 1 to 4)
-            const float d = -(float)max(n, 1), rd = -1.0f / d;
+            // s / n, n = 1 to 4: by a power of two it is the product with the exact reciprocal, and by three a
+            // division (cells with one invalid patch).  2048 x 2048, 32 x 32: 154 us, with a division throughout 232
+            const float rn = n == 4 ? 0.25f : n == 2 ? 0.5f : 1.f;
             float2* o = a.out + (long long)y0 * a.op + x;
+            auto write = [&](auto quotient) {
 #pragma unroll
-            for (int r = 0; r < SY; r++) {
-                if (y0 + r < a.ny) {
-                    const float2 s = add2(tot[r], exch[((buf * NS + slot - 1) * SY + r) * SX + c]);
-                    const bool bad = n == 0 || ((nan >> r) & 1u);
-                    const float q = __int_as_float(0x7fc00000);
-                    const float2 p = mul2(s, make_float2(rd, rd));
-                    const float2 e = fma2(make_float2(d, d), p, s);
-                    o[(long long)r * a.op] = bad ? make_float2(q, q) : fma2(e, make_float2(rd, rd), p);
+                for (int r = 0; r < SY; r++) {
+                    if (y0 + r < a.ny) {
+                        const float2 s = add2(tot[r], exch[((buf * NS + slot - 1) * SY + r) * SX + c]);
+                        const bool bad = n == 0 || ((nan >> r) & 1u);
+                        const float q = __int_as_float(0x7fc00000);
+                        o[(long long)r * a.op] = bad ? make_float2(q, q) : quotient(s);
+                    }
                 }
-            }
+            };
+            if (n != 3) write([&](float2 s) { return mul2(s, make_float2(rn, rn)); });
+            else write([](float2 s) { return gs_third(s); });
         }
         buf ^= 1;
     }

@@ -138,3 +138,25 @@ def test_cuda_result_in_place_of_the_input():
     _lib.check(lib.unw_goldstein_c64(t.data_ptr(), 170, c.data_ptr(), 170, 150, 170, 16, 16, 0.5, t.data_ptr(), 170,
                                      ws.data_ptr(), ws.numel(), torch.cuda.current_stream(dev).cuda_stream))
     np.testing.assert_array_equal(t.cpu().numpy(), ref)
+
+
+def _impulses(shape, amplitude):
+    """Real impulses in the middle of every second 8 x 8 cell block: each 8 x 8 patch of the interior holds
+    at most one, so its spectrum has the same modulus everywhere."""
+    z = np.zeros(shape, np.complex64)
+    z[6::16, 6::16] = amplitude
+    return z
+
+
+# Coherence 0 makes the power 1: the spectrum of an impulse A becomes A |A| everywhere, and its inverse sum
+# 64 A |A| passes float32 in the last butterfly alone (32 A |A| is below 3.4e38).  The sum is divided by the
+# number of patches as any other: an infinite sum stays infinite, and nothing turns into NaN.
+@pytest.mark.gpu
+def test_cuda_overflowed_sum_stays_infinite():
+    _gpu()
+    import core_b200
+    z = _impulses((48, 64), np.float32(2.5e18))
+    out = core_b200.goldstein(z, np.zeros(z.shape, np.float32), 8, 8, 0.5)
+    at = z != 0
+    assert np.isposinf(out.real[at]).all() and np.isfinite(out.imag[at]).all()
+    assert np.isfinite(out[~at]).all()
