@@ -117,15 +117,16 @@ __device__ __forceinline__ void gs_dit(float2* v) {
     }
 }
 
-// F * max(|F|, 1e-10)^alpha, t = alpha / 2.  The power as 2^(t log2 |F|^2) with the exponent e of |F|^2
-// kept apart from its mantissa f: t e is split into its nearest integer n and an exact rest, so
-// what the units' log2 and exp2 see stays below 1 and their error (2^-22.6 absolute of log2 f,
-// times t <= 1/2; 2 ulp of exp2) does not grow with |F|.  Measured against 64 bits over a filtered
-// grid: 1.7e-7, with powf(sqrtf) 1.8e-7.  For |t| <= 1; |F|^2 beyond float32 is taken as its
-// largest value.
+// F * max(|F|, 1e-10)^alpha, t = alpha / 2, as 2^(t log2 |F|^2) with the argument split into an integer and a
+// rest (W. J. Cody and W. Waite, Software Manual for the Elementary Functions, 1980, the chapter on x**y;
+// rounding to the nearest integer by adding 1.5 * 2^23): |F|^2 = 2^e f with sqrt(1/2) <= f < sqrt(2), t e =
+// n + rest, the rest exact by the fma.  The units' log2 and exp2 only see |log2 f| <= 1/2 and a power within
+// [-1, 1], so their error (2^-22.6 absolute of log2 f, times |t| <= 1; 2^-22 of exp2) does not grow with
+// |F|.  Measured against 64 bits over a filtered grid: 1.7e-7, with powf(sqrtf) 1.8e-7.
+// For |t| <= 1 and |F.x|, |F.y| < 2^62: |F|^2 <= 2^125, so that 2^n is a normal number.
 __device__ __forceinline__ float2 gs_weight(float2 F, float t) {
     constexpr float magic = 12582912.f;                     // 1.5 * 2^23: integers in the low bits
-    const float m2 = fminf(fmaxf(fmaf(F.x, F.x, F.y * F.y), 1e-20f), 3e38f);
+    const float m2 = fmaxf(fmaf(F.x, F.x, F.y * F.y), 1e-20f);
     const int e = (__float_as_int(m2) - 0x3f3504f3) >> 23;  // mantissa in [0.707, 1.414)
     const float f = __int_as_float(__float_as_int(m2) - (e << 23));
     const float fe = __int_as_float(0x4b400000 + e) - magic;
@@ -136,9 +137,14 @@ __device__ __forceinline__ float2 gs_weight(float2 F, float t) {
     const float s = x * __int_as_float((__float_as_int(nm) << 23) + 0x3f800000);
     return mul2(F, make_float2(s, s));
 }
-// the same for any alpha (coherence outside [0, 1])
+// The same for any alpha (coherence outside [-1, 3]) and any |F| (scaled by a power of two where its square
+// would overflow).
+constexpr float GS_BIG = 4611686018427387904.f;             // 2^62
 __device__ __noinline__ float gs_pow(float2 F, float alpha) {
-    return powf(fmaxf(sqrtf(F.x * F.x + F.y * F.y), 1e-10f), alpha);
+    const bool big = fmaxf(fabsf(F.x), fabsf(F.y)) >= GS_BIG;
+    if (big) F = make_float2(F.x * 0x1p-66f, F.y * 0x1p-66f);
+    const float m = sqrtf(F.x * F.x + F.y * F.y);
+    return powf(fmaxf(big ? m * 0x1p66f : m, 1e-10f), alpha);
 }
 
 __device__ __noinline__ float2 gs_third(float2 s) { return make_float2(s.x / 3.f, s.y / 3.f); }
@@ -260,7 +266,10 @@ __global__ void __launch_bounds__(256, (GsShape<PY, PX>::CTAS)) k_gs_walk(GsArgs
                 for (int k = 0; k < PX; k++) u[k] = tile[r * (PX + 1) + k];
                 gs_dif<PX>(u);
                 // spectrum weight (:270-276)
-                if (fabsf(alpha) <= 2.f) {
+                float top = 0.f;
+#pragma unroll
+                for (int k = 0; k < PX; k++) top = fmaxf(top, fmaxf(fabsf(u[k].x), fabsf(u[k].y)));
+                if (fabsf(alpha) <= 2.f && top < GS_BIG) {
 #pragma unroll
                     for (int k = 0; k < PX; k++) u[k] = gs_weight(u[k], 0.5f * alpha);
                 } else {

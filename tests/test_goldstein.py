@@ -160,3 +160,32 @@ def test_cuda_overflowed_sum_stays_infinite():
     at = z != 0
     assert np.isposinf(out.real[at]).all() and np.isfinite(out.imag[at]).all()
     assert np.isfinite(out[~at]).all()
+
+
+# The spectrum weight max(|F|, 1e-10)^alpha by itself, against the float64 power: an impulse A of weight 1 in its
+# patches comes out as A max(A, 1e-10)^alpha times the mean of the four tapers over it.  Coherence c (constant)
+# gives alpha = 1 - c, outside [0, 1] too, |alpha| <= 2 and beyond (where the general form runs), and A goes from
+# below the floor of 1e-10 to moduli whose square is beyond float32.  Relative tolerance, from the
+# operations' bounds: 4e-6 for twelve butterfly stages (3.8 u each, u = 2^-24) and the power itself, and 8e-7 |c|
+# for alpha (11 additions of the weighted coherence and two roundings) times |ln A|, which the power multiplies it by.
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", [0.0, 0.5, 1.0, 0.96875, -0.75, -1.0, 1.75, 3.0, -1.5, 4.5])
+@pytest.mark.parametrize("amp", [3e-12, 1e-10, 7.3e-8, 1e-4, 0.711, 1.0, 1.413, 37.0, 1e6, 2.2e12, 3.1e18, 4.7e18, 1.6e19,
+                                 1.9e19, 1e20, 2.5e24])
+def test_cuda_spectrum_weight_of_an_impulse(c, amp):
+    _gpu()
+    import core_b200
+    z = _impulses((48, 64), np.float32(amp))
+    A = float(np.float32(amp))
+    F = A * max(A, 1e-10) ** (1.0 - c)
+    held = A * float(np.float32(max(A, 1e-10) ** (1.0 - c)))   # the power is a float32 (zero below 1e-45)
+    if not 1e-30 < F < 1e36:
+        pytest.skip("the weighted spectrum, or its sum, is outside float32")
+    out = core_b200.goldstein(z, np.full(z.shape, c, np.float32), 8, 8, 0.5)
+    taper = 1.0 - abs(np.array([2.0, 1.0]) - 3.0) / 3.0   # local rows 2 and 6 (mirrored: 1)
+    ref = held * np.outer(taper, taper).sum() / 4
+    # impulses whose four patches lie inside the grid (beyond it the coherence is 0)
+    at = [(y, x) for y in (6, 22, 38) for x in (6, 22, 38, 54)]
+    got = np.array([out[p] for p in at])
+    tol = 4e-6 + 8e-7 * abs(c) * abs(np.log(A))
+    assert np.abs(got - ref).max() <= tol * ref
