@@ -108,10 +108,16 @@ __global__ void k_state_init(const GridDev* __restrict__ grids, int n, UnwScalar
 // NaN fill, weight clipping, wrapped gradients and edge weights
 // (utils_unwrap2d.py:1228-1241, :1254-1262, :1267-1275).  KS_ELEM shape.
 //
-// atan2(sin d, cos d) as d - 2 pi k with the nearest integer k in float64, rounded once: within half an
-// ulp of the wrapped difference where the three float32 functions lose several, and the kernel,
-// which they bounded (with a 64-bit division per pixel), 300 -> 190 us at 4096 x 4096.
-__device__ __forceinline__ float wrap_f(float d) {
+// atan2(sin d, cos d) as d - 2 pi k with the nearest integer k in float64 and 2 pi in two parts (the
+// reduction of W. J. Cody and W. Waite, Software Manual for the Elementary Functions, 1980), rounded once: within
+// half an ulp of the wrapped difference where the three float32 functions lose several, and the kernel, which they
+// bounded (with a 64-bit division per pixel), 290 -> 183 us at 4096 x 4096.  Up to |d| = 1e8 the integer is off the
+// nearest by less than 4e-9 of a cycle, which leaves the result within fl(pi).  Beyond, it is no longer resolved
+// (from 1e16 on by whole cycles) and the functions' own reduction is taken, in a loop of its own (2% of the kernel;
+// as a call per difference 5%).  Four CTAs per SM: with the 68 registers of an unbounded kernel three are
+// resident and it takes 246 us.
+constexpr float WRAP_NEAR = 1e8f;
+__device__ __forceinline__ float wrap_near(float d) {
     const double x = (double)d, k = rint(x * 0.15915494309189535);
     return (float)fma(k, -2.4492935982947064e-16, fma(k, -6.283185307179586, x));
 }
@@ -129,7 +135,7 @@ __device__ __forceinline__ void px_in(const GridDev& G, int i, int j, float& ph,
     }
 }
 
-__global__ void k_setup(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
+__global__ void __launch_bounds__(256, 4) k_setup(const GridDev* __restrict__ grids, const int* __restrict__ starts, int n) {
     __shared__ double red[32 * 1];
     const int g = find_grid(starts, n, blockIdx.x);
     const GridDev& G = grids[g];
@@ -137,6 +143,7 @@ __global__ void k_setup(const GridDev* __restrict__ grids, const int* __restrict
     const int nct = starts[g + 1] - starts[g];
     const int H = G.H, W = G.W, P = G.P;
     double acc[1] = {0.0};
+    bool far = false;
     UNW_PIECES_LOOP(G, local, nct, 1) {
         float ph, w, phr, wr, phd, wd;
         bool v, vr, vd;
@@ -144,18 +151,35 @@ __global__ void k_setup(const GridDev* __restrict__ grids, const int* __restrict
         float gxv = 0.f, wxv = 0.f, gyv = 0.f, wyv = 0.f;
         if (j < W - 1) {
             px_in(G, i, j + 1, phr, wr, vr);
-            gxv = wrap_f(fsub(phr, ph));
+            const float d = fsub(phr, ph);
+            far |= fabsf(d) > WRAP_NEAR;
+            gxv = wrap_near(d);
             wxv = fmul(fdiv(fadd(w, wr), 2.0f), (v && vr) ? 1.f : 0.f);
         }
         if (i < H - 1) {
             px_in(G, i + 1, j, phd, wd, vd);
-            gyv = wrap_f(fsub(phd, ph));
+            const float d = fsub(phd, ph);
+            far |= fabsf(d) > WRAP_NEAR;
+            gyv = wrap_near(d);
             wyv = fmul(fdiv(fadd(w, wd), 2.0f), (v && vd) ? 1.f : 0.f);
         }
         const size_t o = (size_t)i * P + j;
         G.gx[o] = gxv; G.gy[o] = gyv; G.wx[o] = wxv; G.wy[o] = wyv;
         G.valid[o] = v ? 1 : 0;
         acc[0] += v ? 1.0 : 0.0;
+    }
+    if (far) {  // once more over this thread's pixels, for the differences that wrap_near does not resolve
+        UNW_PIECES_LOOP(G, local, nct, 1) {
+            float ph, w, ph1;
+            bool v;
+            px_in(G, i, j, ph, w, v);
+            for (int y = 0; y < 2; y++) {
+                if (y ? i == H - 1 : j == W - 1) continue;
+                px_in(G, i + y, j + 1 - y, ph1, w, v);
+                const float d = fsub(ph1, ph);
+                if (fabsf(d) > WRAP_NEAR) (y ? G.gy : G.gx)[(size_t)i * P + j] = atan2f(sinf(d), cosf(d));
+            }
+        }
     }
     if (arrive<1>(G, local, nct, acc, red)) {
         finish_sum<1>(G, nct, acc, red);
