@@ -123,3 +123,32 @@ def test_autotuner_reports_its_choice():
     uf, ccf = core_b200.irls_unwrap_2d(p, c)
     v = np.isfinite(p)
     assert (cycle_map(u, p) == cycle_map(uf, p))[v].mean() >= 0.9999
+
+
+def _launches(fn, kernel):
+    """Launches of the kernels whose name holds `kernel` during fn()."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return sum(e.count for e in prof.key_averages() if kernel in e.key)
+
+
+def test_uneven_mixed_batch_shares_launches():
+    # the setup kernel runs once per launch group: heights of one class (here one Bluestein length, or any heights
+    # where the tensor cores are ruled out) form one group as in the plain form; where the tensor-core pass is asked
+    # for, which needs one height per launch, every height has its own
+    sizes = [(300, 300), (311, 300), (322, 290), (333, 310)]
+    grids = [gen_g1(h, w, seed=h)[:2] for h, w in sizes]
+    ps = [torch.from_numpy(p).to(DEV) for p, _ in grids]
+    cs = [torch.from_numpy(c).to(DEV) for _, c in grids]
+    kw = dict(max_iter=2, cg_max_iter=4)
+    plain = core_b200.irls_unwrap_2d_batch(ps, cs, **kw)
+    for col_pass, groups in (("auto", 1), ("fft", 1), ("tc", 4)):
+        run = lambda: core_b200.irls_unwrap_2d_batch(ps, cs, precision="mixed", col_pass=col_pass, return_stats=True, **kw)
+        mixed = run()
+        assert _launches(run, "k_setup") == groups
+        for (u, _, st), (v, _) in zip(mixed, plain):
+            assert st["col_path"] == (col_pass == "tc")
+            if not st["col_path"]:
+                assert torch.equal(u.view(torch.int32), v.view(torch.int32))
