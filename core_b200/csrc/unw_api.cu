@@ -1088,8 +1088,8 @@ int adjoint_group(const std::vector<int>& idx, const unw_adj_grid* grids, const 
     CK(unw_launch_simple(UNW_K_STATE_INIT, 1, s, S.dg, S.ds(KS_ELEM), n, 0, S.sc));
     CK(unw_launch_simple(UNW_K_SETUP, ne, s, S.dg, S.ds(KS_ELEM), n, 0, S.sc));
     CK(unw_launch_adj(UNW_A_LOAD, ne, s, S.dg, S.ds(KS_ELEM), n));
-    // 1. the frozen-weight system at u (IRLS weights and right-hand side from u), solved to
-    //    the relative tolerance from u: u* in U1
+    // 1. the frozen-weight system at u (IRLS weights from u; the PCG start forms b - A u from
+    //    them), solved to the relative tolerance from u: u* in U1
     rc = enqueue_iteration(S, 0, UNW_ADJ_CHUNK);
     if (rc) return rc;
     // 2. iterative refinement of u* on the frozen system: residual in float64 (phase

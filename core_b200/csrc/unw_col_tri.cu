@@ -32,16 +32,16 @@
 //   r.z = sum_i sum_l e_l X_l(i) Z_l(i),  e_0 = 1/2, e_l = 1,  Z_l = z_l / 2W as written.
 //
 // What bounds it (B200): 8 bytes per pixel of T and Tz, at 4096 x 4096 134 MB or 20.5 us at the
-// measured copy rate; it takes 31.5 us there (682 CTAs, two per SM at 64 registers; the latency
-// of the four batches of row loads of a segment is most of a CTA's 10.7 us).  Up to 1024 x 1024 it is
+// measured copy rate; it takes 41 us there in the solver (kernel trace; 42 us from cold L2) and 32 us in mode 0,
+// without r.z (682 CTAs, two per SM at 64 registers; the latency of the four batches of row loads of a
+// segment is most of a CTA's 10.7 us).  Up to 1024 x 1024 it is
 // the chain of one CTA, 5 us, of which the wide CTAs are the longest.  In the solver, CUDA-event
 // times per launch against the column FFTs (two transforms and the spectral step) that it
 // replaced: 4096 x 4096 45.5 us / 89.9, 2048 x 2048 15.6 / 22.9, 1838 x 2750 (Bluestein) 22.9 / 110.6,
 // 1024 x 1024 12.9 / 18.8, 200 x 180 11.4 / 25.1 (about 8 us of each is the event pair).
-// Tried and not kept: all columns in float64 in clusters that exchange the chunk states
-// through distributed shared memory (69 us at 4096 x 4096: start-up, barrier and folding
-// took two thirds of a CTA's time), one column per lane (64 us), an L2 prefetch of the
-// segment's rows (47 us).
+// Tried and not kept, at 4096 x 4096: all columns in float64 in clusters that exchange the chunk states
+// through distributed shared memory (69 us: start-up, barrier and folding took two thirds of a
+// CTA's time), one column per lane (64 us), an L2 prefetch of the segment's rows (47 us).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 

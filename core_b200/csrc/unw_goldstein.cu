@@ -16,7 +16,7 @@
 // one launch, deterministic.
 //
 // What bounds it (B200): instruction issue at two CTAs per SM (128 registers a thread): 3700 warp
-// instructions per 32 x 32 patch at 2.3 per cycle, DRAM at 5%.  2048 x 2048 with 32 x 32 patches takes 150 us
+// instructions per 32 x 32 patch at 2.3 per cycle, DRAM at 5%.  2048 x 2048 with 32 x 32 patches takes 154 us
 // (traffic alone 13 us); the earlier form, radix-2 passes through shared memory with a sincospi per
 // butterfly, four launches and an accumulator in global memory, 765 us.  1001 x 1203 with 16 x 16:
 // 39 us, before 280.  Butterflies as packed additions: 154 us against 166 with scalar ones.

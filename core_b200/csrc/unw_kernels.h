@@ -107,11 +107,11 @@ cudaError_t unw_launch_bbox(const float* phase, long long pitch, int H0, int W0,
 
 // post-processing
 enum {
-    UNW_P_KSTATS = 0,   // non-finite count, min/max cycle count
-    UNW_P_HIST,         // histogram of cycle counts
+    UNW_P_KSTATS = 0,   // non-finite count, range and histogram of the cycle counts
+    UNW_P_HIST,         // histogram from the smallest count, for ranges outside the first one's window
     UNW_P_MEDIAN,       // median -> shift (one CTA per grid)
-    UNW_P_SHIFT_CCINIT, // apply shift, NaN restore, union-find init
-    UNW_P_UNION,        // union with right/down neighbours
+    UNW_P_SHIFT_CCINIT, // apply shift, NaN restore, union-find init: runs of valid pixels
+    UNW_P_UNION,        // joins runs across piece borders and with overlapping runs of the row below
     UNW_P_FLATTEN,      // root per pixel, roots per tile
     UNW_P_TILESCAN,     // exclusive scan of tile counts (one CTA per grid)
     UNW_P_LABEL,        // compact labels of roots
@@ -124,7 +124,8 @@ cudaError_t unw_launch_post(int which, int nblk, cudaStream_t s, const GridDev* 
                             int n, const UnwScalars& sc, const GridDev* host_grids);
 
 // Per-grid tensor maps of the TMA-staged passes (one 128-byte CUtensorMap each): the
-// column pass's (tensor-core T / p1, or the tridiagonal pass's T) at UNW_MAP_COL, the matvec's three (p, wIx, wIy) at UNW_MAP_MV.
+// column pass's (tensor-core T / p1, or the tridiagonal pass's T) at UNW_MAP_COL, the matvec's
+// three (p, wIx, wIy) at UNW_MAP_MV.
 #define UNW_MAPS_PER_GRID 8
 #define UNW_MAP_BYTES (128 * UNW_MAPS_PER_GRID)
 #define UNW_MAP_COL 0

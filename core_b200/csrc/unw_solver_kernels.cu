@@ -96,8 +96,10 @@ __global__ void k_state_init(const GridDev* __restrict__ grids, int n, UnwScalar
 // Walk of the elementwise kernels (KS_ELEM): a warp takes row pieces of UNW_ELEM_PIECE columns, a lane V
 // adjacent columns per step; P is a multiple of 4, so a group of four starting below W stays in the row.
 // Rows dealt to whole CTAs left most threads of a narrow grid idle and a small grid's CTAs with a
-// dozen rows one after another: 200 x 180, us per launch, then / now: k_mean 10.0 / 5.7, k_rel 12.6 / 7.2; at
-// 1024 x 1024 7.2 / 7.5 and 9.7 / 12.0; bound there and above by the bytes.
+// dozen rows one after another: 200 x 180, us per launch, rows / pieces: k_mean 9.9 / 5.7, k_rel 12.4 / 7.4; 700 x 900
+// 6.8 / 6.8, 9.4 / 9.4.  From 1024 columns on, where a row holds work for a whole CTA, neither is the better
+// one throughout: k_mean, k_rel at 1024 x 1024 6.9 / 7.4, 10.2 / 11.8 and at 4096 x 4096 39.3 / 49.0, 87.5 / 87.8, but
+// 1024 x 1100 8.9 / 8.1, 15.5 / 14.8 and 200 x 7000 10.8 / 7.9, 19.2 / 15.9; of a solve it is below 0.5% either way.
 #define UNW_PIECES_LOOP(G, local, nct, V)                                                                       \
     for (int np_ = ((G).W + UNW_ELEM_PIECE - 1) / UNW_ELEM_PIECE, q_ = (local) * 8 + (int)(threadIdx.x >> 5), i = 0; \
          q_ < (G).H * np_ && ((i = q_ / np_), true); q_ += (nct) * 8)                                           \

@@ -113,7 +113,7 @@ typedef struct unw_stats {
 #define UNW_S_NONFINITE_OUT      4   /* non-finite output: NaN result            */
 #define UNW_S_ALL_NAN            8   /* input all NaN                            */
 #define UNW_S_TC_TIMEOUT        16   /* a TMA-staged column pass (tensor-core or
-                                        power-of-two) gave up waiting on its copies
+                                        tridiagonal) gave up waiting on its copies
                                         (bounded wait); result not valid        */
 
 /* One grid of a batched solve (unw_solve_batch).  Pitches are in elements. */

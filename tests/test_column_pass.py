@@ -3,8 +3,8 @@
 Checked through the operator entry point against the float64 operator idct2(dct2(r) / lambda), with
 the bar of the other preconditioner tests (2e-5 of the largest value: the rows still go
 through float32 transforms), at the sizes where the pass changes form: columns shorter than
-the 64- and 32-row halos, one row, the edges of the 128- / 192- and 384- / 448-row tiles, strips that
-end inside 64 columns, grids of wide columns only, odd widths (no 8-byte pairs), the longest column.
+the 64- and 32-row halos, one row, the edges of the 128- / 192-row tiles (test_column_pass_edges.py has
+those of the 384- / 448-row ones, which larger grids take), strips that end inside 64 columns, grids of wide columns only, odd widths (no 8-byte pairs), the longest column.
 The solver is checked against the float64 oracle: float32 only enters in the stored vectors, so the
 result is float32-close to it.
 """

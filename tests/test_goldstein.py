@@ -178,9 +178,9 @@ def test_cuda_spectrum_weight_of_an_impulse(c, amp):
     z = _impulses((48, 64), np.float32(amp))
     A = float(np.float32(amp))
     F = A * max(A, 1e-10) ** (1.0 - c)
-    held = A * float(np.float32(max(A, 1e-10) ** (1.0 - c)))   # the power is a float32 (zero below 1e-45)
     if not 1e-30 < F < 1e36:
         pytest.skip("the weighted spectrum, or its sum, is outside float32")
+    held = A * float(np.float32(max(A, 1e-10) ** (1.0 - c)))   # the power is a float32 (zero below 1e-45)
     out = core_b200.goldstein(z, np.full(z.shape, c, np.float32), 8, 8, 0.5)
     taper = 1.0 - abs(np.array([2.0, 1.0]) - 3.0) / 3.0   # local rows 2 and 6 (mirrored: 1)
     ref = held * np.outer(taper, taper).sum() / 4

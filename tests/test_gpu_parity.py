@@ -486,8 +486,8 @@ def _solve_flags(p, c, flags, **kw):
 
 @pytest.mark.parametrize("shape", [(256, 256), (200, 300)])
 def test_graph_launches_equal_direct_launches(shape):
-    # the IRLS iterations run as two captured CUDA graphs unless UNW_F_NO_GRAPH is set;
-    # every kernel is deterministic, so both must give identical bits
+    # the PCG iterations run as a captured CUDA graph of five, launched as often as the cap holds it,
+    # unless UNW_F_NO_GRAPH is set; every kernel is deterministic, so both must give identical bits
     p, c, _ = gen_g2(*shape, seed=7)
     u1, c1, s1 = _solve_flags(p, c, 0)
     u2, c2, s2 = _solve_flags(p, c, _lib.UNW_F_NO_GRAPH)
@@ -501,9 +501,9 @@ def test_graph_launches_equal_direct_launches(shape):
 
 @pytest.mark.parametrize("shape", [(4096, 1000), (4096, 3), (4096, 333), (2048, 777), (2048, 2048)])
 def test_tma_column_pass_equals_plain_loads(shape):
-    # at H = 2048 / 4096 the column pass can move its slab by TMA (forced here; by default an
-    # autotuner picks the faster per shape); the arithmetic is the same as the plain-load
-    # pass, so both must give identical bits (and no timeout status)
+    # the column pass can move its tiles by TMA (on request: UNW_F_COL_TMA; the default is plain
+    # loads); the arithmetic is the same as the plain-load pass, so both must give identical
+    # bits (and no timeout status).  All five shapes take segments of 16 rows
     p, c, _ = gen_g1(*shape, seed=11)
     u1, c1, s1 = _solve_flags(p, c, _lib.UNW_F_COL_TMA)
     u2, c2, s2 = _solve_flags(p, c, _lib.UNW_F_COL_NO_TMA)
